@@ -560,6 +560,10 @@ int gqa_prefill(const ncb_gqa *args, void *stream);
  * ascending positions; a row at position 0 starts from a zero state; a segment whose first position is negative is idle.
  * out NULL: only the state is advanced.
  *   delta_step    token by token; seg_first NULL: every row is a segment; keep: also the ring (every row a slot of its own)
+ *   delta_tokens  what every token needs in one launch over all rows, then a walk over the segments, then norm and gate: for
+ *                 segments of several rows, dim and vdim as delta_tokens_supported() takes them. rank_a and rank_g multiples
+ *                 of 16, offsets and ldp of 8; for bf16 a2_rows and g2_rows as below. Scratch, fp32: tok_qk [rows][kv_heads][2]
+ *                 [dim], tok_g [rows][heads][dim], tok_v [rows][heads][vdim], tok_s [rows][heads][2]. Three launches.
  *   delta_chunked bf16, rank_a and rank_g multiples of 16: segments cut into chunks of at most delta_chunk_tokens() rows
  *                 (= chunk; 0: not taken): chunk_first / chunk_count [n_chunks], chunk_within [n_chunks] (rows of the segment
  *                 before the chunk), seg_chunk [n_segments + 1] (a segment's first chunk). a2_rows bf16 [heads][dim][rank_a], g2_rows [heads][vdim][rank_g]. Scratch per (chunk, head): w_terms,
@@ -583,7 +587,10 @@ typedef struct {
     void *w_terms, *kd_terms, *q_terms, *b_terms, *s_terms, *u_terms;
     float *u0, *chunk_decay, *raw;
     int *status;
+    float *tok_qk, *tok_g, *tok_v, *tok_s;
 } ncb_delta;
+int delta_tokens_supported(int dim, int vdim);
+int delta_tokens(const ncb_delta *args, int f32, void *stream);
 int delta_chunk_tokens(int dim, int vdim, int taps, int rank_a, int rank_g);
 int delta_chunked(const ncb_delta *args, void *stream);
 int delta_step(const ncb_delta *args, int f32, void *stream);

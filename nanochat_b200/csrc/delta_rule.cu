@@ -9,6 +9,8 @@
  *   - k_delta_step: token by token. A block (or a cluster of blocks that share the norm's sum through distributed shared
  *     memory) owns a slice of vdim of one head and holds its part of the state in registers for all tokens of the segment. The
  *     decayed state meets k and q in one pass, o = S'^T q + (k . q) u, so a token costs one reduction over the key channels.
+ *   - delta_tokens (float32, short portions; dim <= 256): k_delta_rows does for all rows in parallel what a token needs before its
+ *     turn, k_delta_walk is left with the recurrence, k_delta_gate norms and gates. Everything stays fp32.
  *   - chunks of up to 64 tokens (prompts, bf16 projections, dim <= 256). With G_t the product of the decays since the chunk's
  *     start, S_t = G_t S_0 + sum_(s <= t) (G_t / G_s) k_s u_s^T, and the u of a chunk solve a unit lower triangular system:
  *         (I + A) U = beta (V - (G K) S_0),  A[t][s] = beta_t sum_d k_td k_sd G_td / G_sd  (s < t),
@@ -1090,6 +1092,445 @@ template <int MT> __global__ void __launch_bounds__(OUT_THREADS, 1) k_delta_out(
 
 /* ---- host side -------------------------------------------------------------------------------------------------------- */
 
+/* ---- several tokens of a segment: what a token needs for all rows in parallel, then a walk ----------------------------- */
+
+constexpr int WALK_THREADS = 128, WALK_WARPS = WALK_THREADS / 32;
+constexpr int WALK_TOKENS = 16, WALK_STAGES = 2; /* tokens copied together, and how many such stages */
+constexpr int WALK_DIM = 256;                   /* the most key channels that a walk's registers hold */
+
+__device__ __forceinline__ bool row_runs(const ncb_delta &a, int row) {
+    const int slot = a.conv.slot_map ? a.conv.slot_map[row] : row;
+    return a.conv.pos[row] >= 0 && slot >= 0 && slot < a.conv.n_slots;
+}
+
+/* A warp's run of consecutive rows: which run at all, and which of those have a tap that is not a row of the pass (or more taps
+ * than a lane keeps). */
+struct Run {
+    uint32_t live, special;
+};
+template <int RUN> __device__ __forceinline__ Run run_of(const ncb_delta &a, int row0, int lane) {
+    const int row = row0 + lane;
+    const bool live = lane < RUN && row < a.conv.rows && row_runs(a, row);
+    const bool special = live && (a.conv.taps > CONV_BATCH || place_of(a.conv, row).before < a.conv.taps - 1);
+    return {__ballot_sync(0xffffffffu, live), __ballot_sync(0xffffffffu, special)};
+}
+
+/* Loads that no store of the same kernel waits for or holds back: what they read, the kernel does not write. */
+__device__ __forceinline__ float4 read4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ float4 read4(const bf16 *p) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+__device__ __forceinline__ float2 read2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
+__device__ __forceinline__ uint4 read16(const bf16 *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
+
+/* Four channels of consecutive rows after convolution and silu: weights and older taps stay in registers. */
+template <typename T> struct ConvLane {
+    const T *proj;
+    int ch;
+    bool on;
+    float4 w[CONV_BATCH], old[CONV_BATCH - 1];
+    ConvLane() = default;
+    __device__ __forceinline__ ConvLane(const ncb_delta &a, int row0, int ch, bool on) : proj((const T *)a.conv.proj + ch), ch(ch), on(on) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int back = 0; back < CONV_BATCH; back++)
+            w[back] = on && back < a.conv.taps ? read4(a.conv.w + (size_t)(a.conv.taps - 1 - back) * a.conv.width + ch) : zero;
+#pragma unroll
+        for (int j = 0; j < CONV_BATCH - 1; j++) /* rows before the pass: what is read instead is not used (special rows) */
+            old[j] = on ? read4(proj + (size_t)max(row0 - (CONV_BATCH - 1) + j, 0) * a.conv.ldp) : zero;
+    }
+    __device__ __forceinline__ float4 load(const ncb_delta &a, int row) const {
+        return on && row < a.conv.rows ? read4(proj + (size_t)row * a.conv.ldp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ float4 next(const ncb_delta &a, int row, float4 x, bool special) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int back = 0; back < CONV_BATCH; back++) {
+            const float4 c = w[back], u = back ? old[CONV_BATCH - 1 - back] : x;
+            y.x = fmaf(c.x, u.x, y.x), y.y = fmaf(c.y, u.y, y.y), y.z = fmaf(c.z, u.z, y.z), y.w = fmaf(c.w, u.w, y.w);
+        }
+        if (special && on) {
+            const Place at = place_of(a.conv, row);
+            const float2 lo = conv2<T>(a.conv, row, at, ch), hi = conv2<T>(a.conv, row, at, ch + 2);
+            y = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < CONV_BATCH - 1; j++) old[j] = old[j + 1];
+        old[CONV_BATCH - 2] = x;
+        return make_float4(silu<T>(y.x), silu<T>(y.y), silu<T>(y.z), silu<T>(y.w));
+    }
+};
+__device__ __forceinline__ float dot4(float4 x, float4 y, float s) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, s)))); }
+__device__ __forceinline__ float4 scaled(float4 x, float f) { return make_float4(x.x * f, x.y * f, x.z * f, x.w * f); }
+__device__ __forceinline__ float warp_sum(float v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+/* The low-rank products of a tile of rows, y[row][c] = sum_r w[c][r] low[row][r] for columns c of one head, handed to `use(row, c,
+ * y0, y1)` (columns c and c + 1). bf16: a warp takes 16 rows by mma.sync; a 16-byte load covers eight of a lane's depths, operands
+ * share the permutation of the depth, so nothing is staged. The products are turned around in shared memory (`turn`: 16 TURN floats
+ * per warp), so that rows leave as whole lines and the code that uses them is a short loop: unrolled over the accumulators it is
+ * thousands of instructions that a block runs once, and fetching those took longer (38 us) than all else here. w_rows [n][rank]. */
+constexpr int TURN = 64 + 4;
+template <typename F> __device__ __forceinline__ void low_rank_rows(const ncb_delta &a, const bf16 *low, const bf16 *w_rows, int rank, int n, int row0, int lane, float *turn, F use) {
+    const int r = lane >> 2, t = lane & 3;
+    const long long row = row0 + r;
+    const bool first = row < a.conv.rows, second = row + 8 < a.conv.rows;
+    for (int n0 = 0; n0 < n; n0 += 64) {
+        float acc[8][4] = {};
+        for (int k0 = 0; k0 < rank; k0 += 32) {
+            const int k = k0 + 8 * t;
+            const bool on = k < rank;
+            const uint4 zero = make_uint4(0, 0, 0, 0);
+            const uint4 x0 = on && first ? read16(low + (size_t)row * a.conv.ldp + k) : zero;
+            const uint4 x1 = on && second ? read16(low + (size_t)(row + 8) * a.conv.ldp + k) : zero;
+            const uint32_t p0[4] = {x0.x, x1.x, x0.y, x1.y}, p1[4] = {x0.z, x1.z, x0.w, x1.w};
+            uint4 w[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                w[i] = on && n0 + 8 * i < n ? read16(w_rows + (size_t)(n0 + 8 * i + r) * rank + k) : zero;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                mma_bf16(acc[i], p0, w[i].x, w[i].y);
+                mma_bf16(acc[i], p1, w[i].z, w[i].w);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            float *at = turn + r * TURN + 8 * i + 2 * t;
+            *reinterpret_cast<float2 *>(at) = make_float2(acc[i][0], acc[i][1]);
+            *reinterpret_cast<float2 *>(at + 8 * TURN) = make_float2(acc[i][2], acc[i][3]);
+        }
+        __syncwarp();
+        const int c = n0 + 2 * lane;
+#pragma unroll 4
+        for (int i = 0; i < 16; i++)
+            if (row0 + i < a.conv.rows && c < n) {
+                const float2 y = *reinterpret_cast<const float2 *>(turn + i * TURN + 2 * lane);
+                use(row0 + i, c, y.x, y.y);
+            }
+        __syncwarp();
+    }
+}
+/* The same in fp32 arithmetic for the 16 rows of a block: a thread per pair of columns of w [rank][ldw], four depths summed before
+ * they join the running sum. `stage`: [16][LOW_DEPTH] floats of shared memory. */
+constexpr int LOW_DEPTH = 64;
+template <typename F> __device__ __forceinline__ void low_rank_rows_f32(const ncb_delta &a, const float *low, const float *w, int ldw, int rank, int n, int row0, float *stage, F use) {
+    for (int n0 = 0; n0 < n; n0 += WALK_THREADS) {
+        const int c = n0 + threadIdx.x;
+        float acc[16] = {};
+        for (int k0 = 0; k0 < rank; k0 += LOW_DEPTH) {
+            const int depth = min(LOW_DEPTH, rank - k0); /* a multiple of 16 */
+            __syncthreads();
+            for (int i = threadIdx.x; i < 16 * depth; i += WALK_THREADS) {
+                const int r = i / depth, k = i - r * depth;
+                stage[r * LOW_DEPTH + k] = row0 + r < a.conv.rows ? __ldg(low + (size_t)(row0 + r) * a.conv.ldp + k0 + k) : 0.f;
+            }
+            __syncthreads();
+            if (c < n)
+#pragma unroll 4
+                for (int k = 0; k < depth; k += 4) {
+                    float f[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) f[j] = __ldg(w + (size_t)(k0 + k + j) * ldw + c);
+#pragma unroll
+                    for (int r = 0; r < 16; r++) {
+                        const float4 x = *reinterpret_cast<const float4 *>(stage + r * LOW_DEPTH + k);
+                        acc[r] += fmaf(f[0], x.x, fmaf(f[1], x.y, fmaf(f[2], x.z, f[3] * x.w)));
+                    }
+                }
+        }
+        if (c < n)
+#pragma unroll
+            for (int r = 0; r < 16; r++)
+                if (row0 + r < a.conv.rows) use(row0 + r, c, acc[r]);
+    }
+}
+
+template <typename T> __host__ __device__ constexpr int walk_run() { return sizeof(T) == 2 ? 16 : 4; } /* rows per warp of the kernels around the walk */
+
+/* Grid (rows / (4 runs) rounded up, kv heads + heads x pieces of 128 values + heads): by unit the unit vectors q, k of a key head,
+ * 128 of a head's values, or a head's decays, in fp32 to tok_qk [row][kv head][2][dim], tok_v [row][head][vdim], tok_g
+ * [row][head][dim]; tok_s [row][head][2] = beta, q . k. Every projected value is loaded once (a lane keeps the older taps), so the
+ * kernel is bound by the fp32 rows that it writes. NC: groups of 128 key channels. */
+template <typename T, int NC> __global__ void __launch_bounds__(WALK_THREADS) k_delta_rows(const ncb_delta a) {
+    constexpr int RUN = walk_run<T>(), BATCH = 4;
+    __shared__ __align__(16) float stage[sizeof(T) == 2 ? WALK_WARPS * 16 * TURN : 16 * LOW_DEPTH];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile0 = blockIdx.x * (WALK_WARPS * RUN), row0 = tile0 + warp * RUN;
+    const int H = a.heads, G = a.kv_heads, D = a.dim, V = a.vdim, pieces = (V + 127) / 128;
+    const long long rows = a.conv.rows;
+    int unit = blockIdx.y;
+    if (unit < G) {
+        const Run run = run_of<RUN>(a, row0, lane);
+        if (!run.live) return;
+        ConvLane<T> q[NC], k[NC];
+#pragma unroll
+        for (int j = 0; j < NC; j++) {
+            const int c = 128 * j + 4 * lane;
+            q[j] = ConvLane<T>(a, row0, a.off_q + unit * D + c, c < D), k[j] = ConvLane<T>(a, row0, a.off_k + unit * D + c, c < D);
+        }
+        float *to = a.tok_qk + ((size_t)row0 * G + unit) * 2 * D;
+#pragma unroll 1
+        for (int r0 = 0; r0 < RUN && row0 + r0 < rows; r0 += BATCH) {
+            float4 xq[BATCH][NC], xk[BATCH][NC];
+#pragma unroll
+            for (int e = 0; e < BATCH; e++)
+#pragma unroll
+                for (int j = 0; j < NC; j++) xq[e][j] = q[j].load(a, row0 + r0 + e), xk[e][j] = k[j].load(a, row0 + r0 + e);
+#pragma unroll
+            for (int e = 0; e < BATCH; e++) {
+                const int r = r0 + e, row = row0 + r;
+                const bool special = run.special >> r & 1;
+                float qq = 0.f, kk = 0.f, qk = 0.f;
+#pragma unroll
+                for (int j = 0; j < NC; j++) {
+                    xq[e][j] = q[j].next(a, row, xq[e][j], special), xk[e][j] = k[j].next(a, row, xk[e][j], special);
+                    qq = dot4(xq[e][j], xq[e][j], qq), kk = dot4(xk[e][j], xk[e][j], kk), qk = dot4(xq[e][j], xk[e][j], qk);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) { /* three chains side by side */
+                    const float x = __shfl_xor_sync(0xffffffffu, qq, o), y = __shfl_xor_sync(0xffffffffu, kk, o), z = __shfl_xor_sync(0xffffffffu, qk, o);
+                    qq += x, kk += y, qk += z;
+                }
+                const float qr = a.q_scale / sqrtf(qq + UNIT_EPS), kr = 1.f / sqrtf(kk + UNIT_EPS);
+                if (!(run.live >> r & 1)) continue;
+                float *out = to + (size_t)r * G * 2 * D;
+#pragma unroll
+                for (int j = 0; j < NC; j++)
+                    if (q[j].on) store4(out + 128 * j + 4 * lane, scaled(xq[e][j], qr)), store4(out + D + 128 * j + 4 * lane, scaled(xk[e][j], kr));
+                for (int i = lane; i < H / G; i += 32) a.tok_s[((size_t)row * H + unit * (H / G) + i) * 2 + 1] = qk * qr * kr;
+            }
+        }
+        return;
+    }
+    unit -= G;
+    if (unit < H * pieces) {
+        const Run run = run_of<RUN>(a, row0, lane);
+        if (!run.live) return;
+        const int h = unit / pieces, c = (unit - h * pieces) * 128 + 4 * lane;
+        ConvLane<T> v(a, row0, a.off_v + h * V + c, c < V);
+        if (unit == h * pieces && (run.live >> lane & 1))
+            a.tok_s[((size_t)(row0 + lane) * H + h) * 2] = sigmoid(to_f(((const T *)a.conv.proj)[(size_t)(row0 + lane) * a.conv.ldp + a.off_b + h]));
+        float *to = a.tok_v + ((size_t)row0 * H + h) * V + c;
+#pragma unroll 1
+        for (int r0 = 0; r0 < RUN && row0 + r0 < rows; r0 += BATCH) {
+            float4 x[BATCH];
+#pragma unroll
+            for (int e = 0; e < BATCH; e++) x[e] = v.load(a, row0 + r0 + e);
+#pragma unroll
+            for (int e = 0; e < BATCH; e++) {
+                const float4 y = v.next(a, row0 + r0 + e, x[e], run.special >> (r0 + e) & 1);
+                if ((run.live >> (r0 + e) & 1) && v.on) store4(to + (size_t)(r0 + e) * H * V, y);
+            }
+        }
+        return;
+    }
+    const int h = unit - H * pieces;
+    const float a_exp = a.a_exp[h], *bias = a.dt_bias + h * D;
+    float *g = a.tok_g + (size_t)h * D;
+    const T *low = (const T *)a.conv.proj + a.off_a;
+    if constexpr (sizeof(T) == 2)
+        low_rank_rows(a, low, (const bf16 *)a.a2_rows + (size_t)h * D * a.rank_a, a.rank_a, D, row0, lane, stage + warp * 16 * TURN, [&](int row, int c, float x, float y) {
+            const float2 b = read2(bias + c);
+            *reinterpret_cast<float2 *>(g + (size_t)row * H * D + c) = make_float2(decay_of<T>(x + b.x, a_exp), decay_of<T>(y + b.y, a_exp));
+        });
+    else
+        low_rank_rows_f32(a, low, (const float *)a.a2 + (size_t)h * a.rank_a * D, D, a.rank_a, D, tile0, stage, [&](int row, int c, float x) {
+            g[(size_t)row * H * D + c] = decay_of<T>(x + __ldg(bias + c), a_exp);
+        });
+}
+
+/* Floats of one token in a walk's stage: k, q, g (each padded to what a lane loads), the block's values, beta and q . k. */
+__host__ __device__ constexpr int walk_record(int NI, int columns) { return 3 * 64 * NI + columns + 4; }
+
+/* The recurrence of one segment and head over a block's slice of the values, the state in registers: 16 lanes share the key
+ * channels (4 NI each), a lane holds CW values, so a warp holds 2 CW. The decayed state meets k and q in one pass; the 2 CW sums are
+ * halved over the 16 lanes, so one of them ends with one sum each. What the tokens need comes through a ring of cp.async stages;
+ * the only barriers are the stages'. o replaces v in tok_v. Bound by the four fp32 operations per state element and token while
+ * many segments are in flight, by a token's chain (products, four shuffle rounds, one broadcast) for a single one: 0.21 us a token
+ * (6 heads of 128 x 128, fp32), where k_delta_step, whose chain goes through the convolution, three block-wide sums and the
+ * low-rank products, takes 11.5. */
+template <int NI, int CW> __global__ void __launch_bounds__(WALK_THREADS) k_delta_walk(const ncb_delta a) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int COLS = 2 * CW * WALK_WARPS, REC = walk_record(NI, COLS), DP = 64 * NI;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, dl = lane & 15, half = lane >> 4;
+    const int h = blockIdx.y, D = a.dim, V = a.vdim, H = a.heads, G = a.kv_heads, kvh = h / (H / G), block0 = blockIdx.x * COLS;
+    const int first = a.seg_first[blockIdx.z], count = a.seg_count[blockIdx.z];
+    const int pos0 = a.conv.pos[first], slot = a.conv.slot_map ? a.conv.slot_map[first] : first;
+    const bool bad = pos0 >= 0 && (slot < 0 || slot >= a.conv.n_slots);
+    const int c0 = block0 + (warp * 2 + half) * CW; /* this lane's first value */
+    float *state = a.state + ((size_t)(bad || slot < 0 ? 0 : slot) * H + h) * D * V + c0;
+    /* positions, slots and the state were written before the launch this one depends on, so the state starts towards registers */
+    float2 s[CW][2 * NI];
+#pragma unroll
+    for (int i = 0; i < 2 * NI; i++) {
+        const int d = 64 * (i / 2) + 4 * dl + 2 * (i & 1);
+#pragma unroll
+        for (int c = 0; c < CW; c++) {
+            const bool on = pos0 > 0 && !bad && d < D && c0 + c < V;
+            s[c][i] = on ? make_float2(state[(size_t)d * V + c], state[(size_t)(d + 1) * V + c]) : make_float2(0.f, 0.f);
+        }
+    }
+    for (int i = tid; i < WALK_STAGES * WALK_TOKENS * REC; i += WALK_THREADS) sm[i] = 0.f; /* channels past dim, values past vdim */
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (bad && tid == 0) flag(a.status, NCB_DEV_BAD_POSITION);
+    if (pos0 < 0 || bad) return;
+    __syncthreads();
+    const int per = D / 4, values = min(COLS, V - block0) / 4, chunks = 3 * per + values + 1;
+    auto fetch = [&](int t0) { /* tokens t0 .. into their stage */
+        float *stage = sm + t0 / WALK_TOKENS % WALK_STAGES * (WALK_TOKENS * REC);
+        const int n = min(WALK_TOKENS, count - t0);
+        for (int i = tid; i < chunks && n > 0; i += WALK_THREADS) {
+            const int which = i < 3 * per ? i / per : 3, j = i - which * per;
+            const size_t row = first + t0;
+            const float *src;
+            int step, at;
+            if (which < 2) src = a.tok_qk + ((row * G + kvh) * 2 + (which ^ 1)) * D + 4 * j, step = 2 * G * D, at = which * DP + 4 * j;
+            else if (which == 2) src = a.tok_g + (row * H + h) * D + 4 * j, step = H * D, at = 2 * DP + 4 * j;
+            else if (j < values) src = a.tok_v + (row * H + h) * V + block0 + 4 * j, step = H * V, at = 3 * DP + 4 * j;
+            else {
+                for (int t = 0; t < n; t++)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(stage + t * REC + 3 * DP + COLS)), "l"(a.tok_s + ((row + t) * H + h) * 2) : "memory");
+                continue;
+            }
+            for (int t = 0; t < n; t++) cp_async16(smem_addr(stage + t * REC + at), src + (size_t)t * step);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < WALK_STAGES - 1; i++) fetch(i * WALK_TOKENS);
+    /* which of the 2 CW sums this lane ends with: o for the upper eight lanes, and of which value */
+    const bool is_o = dl & 8;
+    const int mine = CW == 4 ? dl >> 1 & 3 : CW == 2 ? dl >> 2 & 1 : 0;
+    constexpr int SPARE = CW == 4 ? 1 : CW == 2 ? 3 : 7; /* lanes that hold the same sum */
+    const bool writes = is_o && !(dl & SPARE) && c0 + mine < V;
+    float *out = a.tok_v + ((size_t)first * H + h) * V + c0 + mine;
+    for (int t0 = 0; t0 < count; t0 += WALK_TOKENS) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(WALK_STAGES - 2) : "memory");
+        __syncthreads(); /* the stage has landed, and everybody has left the one that is filled next */
+        fetch(t0 + (WALK_STAGES - 1) * WALK_TOKENS);
+        const float *rec = sm + t0 / WALK_TOKENS % WALK_STAGES * (WALK_TOKENS * REC);
+        const int n = min(WALK_TOKENS, count - t0);
+        struct Operands { /* of one token, as pairs of channels */
+            float2 k[2 * NI], q[2 * NI], g[2 * NI], bq;
+            float v;
+        };
+        auto load = [&](const float *p, Operands &x) {
+#pragma unroll
+            for (int i = 0; i < NI; i++) {
+                const float4 *at = reinterpret_cast<const float4 *>(p + 64 * i + 4 * dl);
+                *reinterpret_cast<float4 *>(x.k + 2 * i) = at[0], *reinterpret_cast<float4 *>(x.q + 2 * i) = at[DP / 4], *reinterpret_cast<float4 *>(x.g + 2 * i) = at[DP / 2];
+            }
+            x.v = p[3 * DP + (warp * 2 + half) * CW + mine];
+            x.bq = *reinterpret_cast<const float2 *>(p + 3 * DP + COLS);
+        };
+        auto step = [&](const Operands &now, Operands &next, const float *then) {
+            float2 x[CW], y[CW];
+#pragma unroll
+            for (int c = 0; c < CW; c++) x[c] = y[c] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 2 * NI; i++)
+#pragma unroll
+                for (int c = 0; c < CW; c++) {
+                    s[c][i] = mul2(s[c][i], now.g[i]);
+                    x[c] = fma2(now.k[i], s[c][i], x[c]);
+                    y[c] = fma2(now.q[i], s[c][i], y[c]);
+                }
+            load(then, next);
+            float z[2 * CW]; /* S'^T k of the lane's values, then S'^T q */
+#pragma unroll
+            for (int c = 0; c < CW; c++) z[c] = x[c].x + x[c].y, z[CW + c] = y[c].x + y[c].y;
+#pragma unroll
+            for (int off = 8, m = CW; off > 0; off >>= 1, m >>= 1) {
+                if (m == 0) z[0] += __shfl_xor_sync(0xffffffffu, z[0], off);
+                const bool upper = dl & off;
+#pragma unroll
+                for (int i = 0; i < CW; i++)
+                    if (i < m) {
+                        const float keep = upper ? z[i + m] : z[i], give = upper ? z[i] : z[i + m];
+                        z[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+                    }
+            }
+            const float u = now.bq.x * (now.v - z[0]); /* of use in the lower eight lanes */
+            const float below = __shfl_xor_sync(0xffffffffu, u, 8);
+#pragma unroll
+            for (int c = 0; c < CW; c++) {
+                const float uc = __shfl_sync(0xffffffffu, u, (lane & 16) | c * (8 / CW));
+                const float2 uu = make_float2(uc, uc);
+#pragma unroll
+                for (int i = 0; i < 2 * NI; i++) s[c][i] = fma2(now.k[i], uu, s[c][i]);
+            }
+            if (writes) *out = fmaf(now.bq.y, below, z[0]);
+            out += (size_t)H * V;
+        };
+        Operands even, odd;
+        load(rec, even);
+#pragma unroll 1
+        for (int t = 0; t < n; t += 2, rec += 2 * REC) { /* what is loaded past the last token lies in the ring and is not used */
+            step(even, odd, rec + (t + 1 < n ? REC : 0));
+            if (t + 1 < n) step(odd, even, rec + (t + 2 < n ? 2 * REC : 0));
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 2 * NI; i++) {
+        const int d = 64 * (i / 2) + 4 * dl + 2 * (i & 1);
+#pragma unroll
+        for (int c = 0; c < CW; c++)
+            if (d < D && c0 + c < V) state[(size_t)d * V + c] = s[c][i].x, state[(size_t)(d + 1) * V + c] = s[c][i].y;
+    }
+}
+
+/* Grid (rows / (4 runs) rounded up, heads): norm of o over a head's values, weight, and the low-rank gate. */
+template <typename T> __global__ void __launch_bounds__(WALK_THREADS) k_delta_gate(const ncb_delta a) {
+    constexpr int RUN = walk_run<T>();
+    __shared__ __align__(16) float stage[sizeof(T) == 2 ? WALK_WARPS * 16 * TURN : 16 * LOW_DEPTH];
+    __shared__ float rstd[WALK_WARPS * RUN]; /* below 0: the row does not run, its output is zero */
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tile0 = blockIdx.x * (WALK_WARPS * RUN), row0 = tile0 + warp * RUN;
+    const int h = blockIdx.y, H = a.heads, V = a.vdim;
+    const float *raw = a.tok_v + (size_t)h * V;
+    const uint32_t live = __ballot_sync(0xffffffffu, lane < RUN && row0 + lane < a.conv.rows && row_runs(a, row0 + lane));
+    float mine = 0.f; /* lane r: the sum of row r */
+    for (int r0 = 0; r0 < RUN; r0 += 4) {
+        float sum[4] = {};
+        for (int c = 4 * lane; c < V; c += 128)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (live >> (r0 + e) & 1) {
+                    const float4 x = read4(raw + (size_t)(row0 + r0 + e) * H * V + c);
+                    sum[e] = dot4(x, x, sum[e]);
+                }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            sum[e] = warp_sum(sum[e]);
+            if (lane == r0 + e) mine = sum[e];
+        }
+    }
+    if (lane < RUN) rstd[warp * RUN + lane] = live >> lane & 1 ? 1.f / sqrtf(mine / (float)a.norm_count + a.eps) : -1.f;
+    __syncthreads();
+    T *out = (T *)a.out + (size_t)h * V;
+    const T *low = (const T *)a.conv.proj + a.off_g;
+    if constexpr (sizeof(T) == 2)
+        low_rank_rows(a, low, (const bf16 *)a.g2_rows + (size_t)h * V * a.rank_g, a.rank_g, V, row0, lane, stage + warp * 16 * TURN, [&](int row, int c, float x, float y) {
+            const float f = rstd[row - tile0];
+            const float2 o = f < 0.f ? make_float2(0.f, 0.f) : read2(raw + (size_t)row * H * V + c);
+            const float2 w = read2(a.norm + c);
+            store2(out + (size_t)row * a.ldo + c, f < 0.f ? 0.f : o.x * f * w.x * sigmoid(x), f < 0.f ? 0.f : o.y * f * w.y * sigmoid(y));
+        });
+    else
+        low_rank_rows_f32(a, low, (const float *)a.g2 + (size_t)h * a.rank_g * V, V, a.rank_g, V, tile0, stage, [&](int row, int c, float x) {
+            const float f = rstd[row - tile0];
+            out[(size_t)row * a.ldo + c] = f < 0.f ? 0.f : __ldg(raw + (size_t)row * H * V + c) * f * __ldg(a.norm + c) * sigmoid(x);
+        });
+}
+
 int check(const ncb_delta &g) {
     const int rc = check_conv(g.conv);
     if (rc != NCB_OK || g.conv.rows == 0) return rc;
@@ -1119,9 +1560,51 @@ template <int C, int DT> int launch_scan(const ncb_delta &g, cudaStream_t stream
     return launch(k_delta_scan<C, DT>, grid, 32 * warps, (size_t)2 * scan_stage(C, g.dim, 16 * warps) + 16, 1, stream, g);
 }
 
+template <int NI, int CW> int launch_walk(const ncb_delta &g, cudaStream_t stream) {
+    constexpr int columns = 2 * CW * WALK_WARPS;
+    const dim3 grid((g.vdim + columns - 1) / columns, g.heads, g.n_segments);
+    return launch(k_delta_walk<NI, CW>, grid, WALK_THREADS, (size_t)WALK_STAGES * WALK_TOKENS * walk_record(NI, columns) * 4, 1, stream, g);
+}
+/* Values per lane: four share a token's operands best; fewer while that leaves the GPU's warp schedulers idle. */
+template <int NI> int launch_walk(const ncb_delta &g, cudaStream_t stream) {
+    const long long values = (long long)g.vdim * g.heads * g.n_segments; /* a warp holds 2 CW of them */
+    return values >= 8 * 4 * 148 ? launch_walk<NI, 4>(g, stream) : values >= 4 * 4 * 148 ? launch_walk<NI, 2>(g, stream) : launch_walk<NI, 1>(g, stream);
+}
+
 } /* namespace */
 
 extern "C" {
+
+int delta_tokens_supported(int dim, int vdim) { return dim > 0 && dim <= WALK_DIM && dim % 16 == 0 && vdim > 0 && vdim % 16 == 0; }
+
+int delta_tokens(const ncb_delta *g, int f32, void *stream_ptr) {
+    if (!g) return NCB_ERR_ARG;
+    int rc = check(*g);
+    if (rc != NCB_OK || g->conv.rows == 0) return rc;
+    if (!delta_tokens_supported(g->dim, g->vdim) || g->rank_a % 16 || g->rank_g % 16) return NCB_ERR_UNSUPPORTED;
+    if (g->n_segments <= 0 || g->n_segments > 65535 || !g->seg_first || !g->seg_count || !g->tok_qk || !g->tok_g || !g->tok_v || !g->tok_s ||
+        (!f32 && (!g->a2_rows || !g->g2_rows)))
+        return NCB_ERR_ARG;
+    if (((uintptr_t)g->tok_qk | (uintptr_t)g->tok_g | (uintptr_t)g->tok_v | (uintptr_t)g->tok_s | (uintptr_t)g->a2_rows | (uintptr_t)g->g2_rows) % 16 ||
+        (g->off_a | g->off_g | g->off_q | g->off_k | g->off_v | (int)g->conv.ldp | g->conv.width) % 8 || g->ldo % 2 || (uintptr_t)g->out % 4 ||
+        ((uintptr_t)g->norm | (uintptr_t)g->dt_bias) % 8)
+        return NCB_ERR_ALIGN;
+    const cudaStream_t stream = (cudaStream_t)stream_ptr;
+    const int tile = WALK_WARPS * (f32 ? walk_run<float>() : walk_run<bf16>()), pieces = (g->vdim + 127) / 128;
+    const unsigned tiles = (unsigned)((g->conv.rows + tile - 1) / tile);
+    const long long units = (long long)g->kv_heads + (long long)g->heads * (pieces + 1);
+    if (units > 65535) return NCB_ERR_UNSUPPORTED;
+    const dim3 grid(tiles, (unsigned)units);
+    if (g->dim <= 128)
+        rc = f32 ? launch(k_delta_rows<float, 1>, grid, WALK_THREADS, 0, 1, stream, *g) : launch(k_delta_rows<bf16, 1>, grid, WALK_THREADS, 0, 1, stream, *g);
+    else
+        rc = f32 ? launch(k_delta_rows<float, 2>, grid, WALK_THREADS, 0, 1, stream, *g) : launch(k_delta_rows<bf16, 2>, grid, WALK_THREADS, 0, 1, stream, *g);
+    if (rc != NCB_OK) return rc;
+    rc = g->dim <= 64 ? launch_walk<1>(*g, stream) : g->dim <= 128 ? launch_walk<2>(*g, stream) : g->dim <= 192 ? launch_walk<3>(*g, stream) : launch_walk<4>(*g, stream);
+    if (rc != NCB_OK || !g->out) return rc;
+    return f32 ? launch(k_delta_gate<float>, dim3(tiles, g->heads), WALK_THREADS, 0, 1, stream, *g)
+               : launch(k_delta_gate<bf16>, dim3(tiles, g->heads), WALK_THREADS, 0, 1, stream, *g);
+}
 
 /* Tokens per chunk of the chunked form for these (padded) sizes; 0: only the token-by-token form takes them. */
 int delta_chunk_tokens(int dim, int vdim, int taps, int rank_a, int rank_g) {

@@ -306,7 +306,11 @@ class ChannelDelta:
     norm, o."""
 
     kv_from = None
-    CHUNKED_FROM = 24  # shorter segments run token by token
+    # Three forms, by the longest segment (10 heads of 128 x 128, bf16, four segments). Token by token in one launch: 25 us for 2
+    # tokens, 44 for 4, 158 for 16. A walk over rows prepared in parallel, three launches, in 32-bit arithmetic: about 60 us up to 16
+    # tokens, 160 for segments of 7 to 300. Chunks on the tensor cores (bf16 only): 67 us for the latter. float32 (6 heads, one
+    # segment of 300): 3,460 us token by token, 145 as a walk.
+    WALKED_FROM, CHUNKED_FROM = 8, 24
 
     def __init__(self, sizes: dict, tensors: dict, eps: float, columns: int, dtype: torch.dtype, device):
         H, G, D, V = (int(sizes[n]) for n in ("heads", "kv_heads", "dim", "vdim"))
@@ -327,6 +331,7 @@ class ChannelDelta:
         self.g2_rows = pad_to(t["g2"].reshape(H, V, -1), H, self.vdim, self.rank_g).to(dtype)
         self.a2, self.g2 = (w.transpose(1, 2).contiguous() for w in (self.a2_rows, self.g2_rows))
         self.chunk = cuda_library("delta_rule").delta_chunk_tokens(self.dim, self.vdim, self.conv.taps, self.rank_a, self.rank_g) if dtype == torch.bfloat16 else 0
+        self.walks = bool(cuda_library("delta_rule").delta_tokens_supported(self.dim, self.vdim))
         self.dt_bias = pad_to(t["dt_bias"].float().reshape(H, D), H, self.dim).contiguous()
         self.a_exp = t["A_log"].float().exp()
         self.norm = pad_to(t["norm"].float(), self.vdim)
@@ -355,11 +360,20 @@ class ChannelDelta:
         if plan is not None:
             first, count = plan.segments()
             a.seg_first, a.seg_count, a.n_segments = first.data_ptr(), count.data_ptr(), plan.n_segments
-        if plan is None or self.chunk == 0 or plan.longest < self.CHUNKED_FROM:
-            check(lib.delta_step(pointer_to(a), f32, stream()), "delta_step")
-        else:
+        if plan is not None and self.chunk and plan.longest >= self.CHUNKED_FROM:
             self.run_chunked(a, rows)
+        elif plan is not None and self.walks and plan.longest >= self.WALKED_FROM:
+            self.run_walk(a, rows)
+        else:
+            check(lib.delta_step(pointer_to(a), f32, stream()), "delta_step")
         self.conv.keep_tail(a.conv, rows)
+
+    def run_walk(self, a: Delta, rows: Rows) -> None:
+        a.a2_rows, a.g2_rows, n = self.a2_rows.data_ptr(), self.g2_rows.data_ptr(), rows.n
+        for name, size in (("tok_qk", 2 * self.kv_heads * self.dim), ("tok_g", self.heads * self.dim), ("tok_v", self.heads * self.vdim),
+                           ("tok_s", 2 * self.heads)):
+            setattr(a, name, rows.buffer("delta_" + name, n * size, torch.float32, self.device).data_ptr())
+        check(cuda_library("delta_rule").delta_tokens(pointer_to(a), int(self.dtype == torch.float32), stream()), "delta_tokens")
 
     def run_chunked(self, a: Delta, rows: Rows) -> None:
         arrays, n = rows.plan.chunks(self.chunk)

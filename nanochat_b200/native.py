@@ -89,7 +89,8 @@ class Delta(ctypes.Structure):
                [("n_segments", c_int)] + \
                [(n, c_ptr) for n in ("a2_rows", "g2_rows", "seg_chunk", "chunk_first", "chunk_count", "chunk_within")] + \
                [("n_chunks", c_int), ("chunk", c_int)] + \
-               [(n, c_ptr) for n in ("w_terms", "kd_terms", "q_terms", "b_terms", "s_terms", "u_terms", "u0", "chunk_decay", "raw", "status")]
+               [(n, c_ptr) for n in ("w_terms", "kd_terms", "q_terms", "b_terms", "s_terms", "u_terms", "u0", "chunk_decay", "raw", "status",
+                                     "tok_qk", "tok_g", "tok_v", "tok_s")]
 
 
 SIGNATURES = {
@@ -160,6 +161,8 @@ SIGNATURES = {
     },
     "delta_rule": {
         "delta_step": ([c_ptr, c_int, c_ptr], c_int),
+        "delta_tokens_supported": ([c_int] * 2, c_int),
+        "delta_tokens": ([c_ptr, c_int, c_ptr], c_int),
         "delta_chunk_tokens": ([c_int] * 5, c_int),
         "delta_chunked": ([c_ptr, c_ptr], c_int),
     },
