@@ -472,7 +472,9 @@ int gla_chunked(const ncb_gla *args, int f32, void *stream);
  *                  per-head rows [w_uk; w_uv] gives ctx_kv, per head [dim | vdim] at stride dim + vdim
  *   latent_prefill out of row tiles: tile_rows (at most 64) rows from tile_row, the first at position tile_pos of the
  *                  sequence whose context starts at row tile_ctx. List the tiles that reach furthest first. dim + rot at
- *                  most 192, vdim at most 128 (latent_prefill_supported) */
+ *                  most 192, vdim at most 128 (latent_prefill_supported)
+ *   latent_prefill_tiles  the same with at most 128 rows per tile, for latent_prefill_tiles_supported sizes; ctx_rows: rows of ctx_kv
+ *                and ctx_rot. scale positive, ldo a multiple of 8 */
 #define NCB_LATENT_TILE 32
 typedef struct {
     void *proj;
@@ -495,6 +497,8 @@ typedef struct {
 int latent_gather(const ncb_latent *args, void *stream);
 int latent_prefill_supported(int dim, int rot, int vdim);
 int latent_prefill(const ncb_latent *args, void *stream);
+int latent_prefill_tiles_supported(int dim, int rot, int vdim);
+int latent_prefill_tiles(const ncb_latent *args, long long ctx_rows, void *stream);
 int latent_append(const ncb_latent *args, int f32, void *stream);
 int latent_query(const ncb_latent *args, int f32, void *stream);
 int latent_split(const ncb_latent *args, int f32, void *stream);
@@ -529,7 +533,8 @@ int short_conv_tail(const ncb_conv *args, int f32, int *status, void *stream);
  *                [rows][heads][max_chunks][vdim + 4]; max_len bounds every position + 1
  *   gqa_merge    out [rows][ldo] = sigmoid(gate) * merged states
  *   gqa_prefill  out of row tiles, bf16: tile_rows (at most 64) rows from tile_row, the first at position tile_pos. List the
- *                tiles that reach furthest first. For gqa_prefill_supported(dim, vdim) */
+ *                tiles that reach furthest first. For gqa_prefill_supported(dim, vdim)
+ *   gqa_prefill_tiles  the same with at most 128 rows per tile, for gqa_prefill_tiles_supported sizes; scale positive, ldo a multiple of 8 */
 #define NCB_GQA_TILE 16
 typedef struct {
     ncb_conv conv;
@@ -550,6 +555,8 @@ int gqa_split(const ncb_gqa *args, int f32, void *stream);
 int gqa_merge(const ncb_gqa *args, int f32, void *stream);
 int gqa_prefill_supported(int dim, int vdim);
 int gqa_prefill(const ncb_gqa *args, void *stream);
+int gqa_prefill_tiles_supported(int dim, int vdim);
+int gqa_prefill_tiles(const ncb_gqa *args, void *stream);
 
 /* ---- library delta_rule ------------------------------------------------------------------------------------------------
  * Gated delta rule with a decay per key channel (csrc/delta_rule.cu has the recurrence). T as above. Projected rows hold q, k

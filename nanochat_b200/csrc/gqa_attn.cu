@@ -11,12 +11,13 @@
  *     softmax state of its own; the block merges its four. In a decode step it also does what k_gqa_rows does: the copies of
  *     the older positions start before the dependency wait, and the new row goes to the cache and straight to its tile;
  *   - k_gqa_merge: the chunks' un-normalised states (m in log2 units, l, o) and the gate;
- *   - k_gqa_prefill: a tile of a prompt's rows of one query head against the cached keys and values.
+ *   - k_gqa_prefill_tiles: a tile of a prompt's rows of one query head against the cached keys and values on tcgen05, for heads of 64 and
+ *     128; k_gqa_prefill: the same on mma.sync, for other sizes and for short segments.
  * Scores and probabilities are fp32; a probability enters the second product as two bf16 terms (hi + lo), so its weight keeps
  * 16 bits. k_gqa_split_any is the split in plain fp32 arithmetic for any sizes and for T = float.
  */
+#include "attn_tiles.cuh"
 #include "short_conv.cuh"
-#include "umma.cuh"
 
 namespace {
 
@@ -712,6 +713,32 @@ template <int QS, int VN, bool EXACT> __global__ void __launch_bounds__(THREADS,
         }
 }
 
+/* Grid (heads, row tiles): the same for at most att::ROWS rows per tile on tcgen05 (attn_tiles.cuh); dim = 64 KB, vdim = 64 VB. Queries
+ * and the cache are read as matrices of heads * dim and dim + vdim columns. */
+template <int KB, int VB> __global__ void __launch_bounds__(att::THREADS, 2) k_gqa_prefill_tiles(const __grid_constant__ CUtensorMap map_q,
+                                                                                             const __grid_constant__ CUtensorMap map_kv, const ncb_gqa a) {
+    extern __shared__ __align__(128) uint8_t raw[];
+    const int h = blockIdx.x, tile = blockIdx.y;
+    att::attend<KB, VB, att::P_TWO, false>(
+        raw, a.status,
+        [&] {
+            att::Work w = {};
+            const int row0 = a.tile_row[tile], rows = min(a.tile_rows[tile], att::ROWS), pos0 = a.tile_pos[tile];
+            int slot, end;
+            const bool ok = rows > 0 && length_of(a, row0, slot) > 0 && length_of(a, row0 + rows - 1, end) == pos0 + rows; /* flagged by gqa_rows too */
+            w.q = &map_q, w.kv = w.rest = &map_kv, w.q_row = row0, w.q_col = h * KB * 64, w.k_boxes = KB, w.v_col = KB * 64;
+            w.kv_row = ok ? (slot * a.kv_heads + h / (a.heads / a.kv_heads)) * a.capacity : 0;
+            w.pos0 = pos0, w.rows = ok ? rows : 0, w.scale = a.scale * att::LOG2_E;
+            return w;
+        },
+        [&](int r, float, float l, int c, const float *v) {
+            const int row = a.tile_row[tile] + r;
+            const float z = to_f(((const bf16 *)a.conv.proj)[(size_t)row * a.conv.ldp + a.off_g + h]);
+            const float f = 1.f / ((1.f + expf(-z)) * l);
+            att::store32((bf16 *)a.out + (size_t)row * a.ldo + h * VB * 64 + c, v, [&](int) { return f; });
+        });
+}
+
 /* ---- merge and gate --------------------------------------------------------------------------------------------------- */
 
 /* Grid (heads, rows): the chunks' states of a head, its gate. */
@@ -849,6 +876,31 @@ int gqa_prefill(const ncb_gqa *g, void *stream) {
     if (g->dim == 64 && g->vdim == 64) return launch(k_gqa_prefill<4, 4, true>, grid, THREADS, smem, 1, s, *g);
     return g->dim <= 128 ? launch(k_gqa_prefill<8, 8, false>, grid, THREADS, smem, 1, s, *g)
                          : launch(k_gqa_prefill<12, 8, false>, grid, THREADS, smem, 1, s, *g);
+}
+
+/* 1 if gqa_prefill_tiles takes these (padded) sizes. */
+int gqa_prefill_tiles_supported(int dim, int vdim) { return (dim == 64 || dim == 128) && (vdim == 64 || vdim == 128); }
+
+int gqa_prefill_tiles(const ncb_gqa *g, void *stream) {
+    if (!g) return NCB_ERR_ARG;
+    const int rc = check(*g);
+    if (rc != NCB_OK || g->conv.rows == 0 || g->n_tiles == 0) return rc;
+    const long long rows = (long long)g->conv.n_slots * g->kv_heads * g->capacity;
+    if (!gqa_prefill_tiles_supported(g->dim, g->vdim) || rows > 0x7fffffffLL || !(g->scale > 0.f)) return NCB_ERR_UNSUPPORTED;
+    if (!g->q || !g->out || g->ldo < g->heads * g->vdim || !g->tile_row || !g->tile_rows || !g->tile_pos || g->n_tiles < 0 || g->n_tiles > 65535)
+        return NCB_ERR_ARG;
+    if (g->ldo % 8) return NCB_ERR_ALIGN;
+    CUtensorMap q, kv;
+    if (!tensor_map(g->q, (int)g->conv.rows, g->heads * g->dim, att::ROWS, &q) || !tensor_map(g->kv, (int)rows, g->dim + g->vdim, att::KEYS, &kv))
+        return NCB_ERR_LAUNCH;
+    const dim3 grid(g->heads, g->n_tiles);
+    const cudaStream_t s = (cudaStream_t)stream;
+    auto run = [&](auto kernel, size_t smem) { return launch(kernel, grid, att::THREADS, smem, 1, s, q, kv, *g); };
+    if (g->dim == 128)
+        return g->vdim == 128 ? run(k_gqa_prefill_tiles<2, 2>, att::Shape<2, 2, att::P_TWO, false>::SMEM_BYTES)
+                              : run(k_gqa_prefill_tiles<2, 1>, att::Shape<2, 1, att::P_TWO, false>::SMEM_BYTES);
+    return g->vdim == 128 ? run(k_gqa_prefill_tiles<1, 2>, att::Shape<1, 2, att::P_TWO, false>::SMEM_BYTES)
+                          : run(k_gqa_prefill_tiles<1, 1>, att::Shape<1, 1, att::P_TWO, false>::SMEM_BYTES);
 }
 
 } /* extern "C" */

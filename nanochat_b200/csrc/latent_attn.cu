@@ -17,10 +17,11 @@
  *     weight keeps 16 bits. Per (row, head, chunk) an un-normalised state (m in log2 units, l, o);
  *   - k_latent_out: merge of the states, sink, the per-head product with W_uv, gate.
  * Expanded form (prompts): k_latent_append, k_latent_gather (the sequences' latent rows as a matrix, whose product with
- * [W_uk; W_uv] is an ordinary GEMM) and k_latent_prefill: a tile of a prompt's rows against the expanded keys and values.
+ * [W_uk; W_uv] is an ordinary GEMM) and a tile of a prompt's rows against the expanded keys and values: k_latent_prefill_tiles (tcgen05,
+ * parts of 64 and 128) or k_latent_prefill (mma.sync, other sizes and short segments).
  * k_latent_split_any and k_latent_out_any are the same steps in plain fp32 arithmetic for any sizes and for T = float.
  */
-#include "umma.cuh"
+#include "attn_tiles.cuh"
 
 #include <cooperative_groups.h>
 
@@ -795,6 +796,43 @@ template <int QS, int VN, bool EXACT> __global__ void __launch_bounds__(THREADS,
                     }
 }
 
+/* Grid (heads, row tiles): the same for at most att::ROWS rows per tile on tcgen05 (attn_tiles.cuh); dim = 64 KA, dim + rot = 64 KB,
+ * vdim = 64 VB. The projection, the expanded keys and values and the rotated parts are read as matrices. */
+template <int KA, int KB, int VB> __global__ void __launch_bounds__(att::THREADS, 2)
+k_latent_prefill_tiles(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_rot,
+                       const ncb_latent a) {
+    extern __shared__ __align__(128) uint8_t raw[];
+    const int h = blockIdx.x, tile = blockIdx.y;
+    att::attend<KB, VB, att::P_TWO, false>(
+        raw, a.status,
+        [&] {
+            att::Work w = {};
+            w.q = &map_q, w.kv = &map_kv, w.rest = &map_rot, w.q_row = a.tile_row[tile], w.q_col = a.off_q + h * KB * 64;
+            w.kv_row = a.tile_ctx[tile], w.k_col = h * (KA + VB) * 64, w.v_col = w.k_col + KA * 64, w.k_boxes = KA;
+            w.pos0 = a.tile_pos[tile], w.rows = min(a.tile_rows[tile], att::ROWS), w.scale = a.scale * att::LOG2_E;
+            return w;
+        },
+        [&](int r, float m, float l, int c, const float *v) {
+            const size_t row = (size_t)a.tile_row[tile] + r;
+            float f = 1.f;
+            if (a.sink) {
+                const float sink = a.sink[h] * LOG2E, top = fmaxf(m, sink);
+                f = exp2f(m - top);
+                l = fmaf(l, f, exp2f(sink - top));
+            }
+            f /= l;
+            const int at = h * VB * 64 + c;
+            uint4 z[4];
+            if (a.gated) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) z[j] = reinterpret_cast<const uint4 *>((const bf16 *)a.proj + row * a.ldp + a.off_g + at)[j];
+            }
+            att::store32((bf16 *)a.out + row * a.ldo + at, v, [&](int j) {
+                return a.gated ? f / (1.f + expf(-__bfloat162float(reinterpret_cast<const bf16 *>(z)[j]))) : f;
+            });
+        });
+}
+
 /* ---- host side ------------------------------------------------------------------------------------------------------ */
 
 template <typename... A>
@@ -930,6 +968,34 @@ int latent_prefill(const ncb_latent *g, void *stream) {
     if (g->dim + g->rot == 192 && g->vdim == 128) return launch(k_latent_prefill<12, 8, true>, grid, smem, THREADS, 1, s, *g);
     return g->dim + g->rot <= 128 ? launch(k_latent_prefill<8, 8, false>, grid, smem, THREADS, 1, s, *g)
                                   : launch(k_latent_prefill<12, 8, false>, grid, smem, THREADS, 1, s, *g);
+}
+
+/* 1 if latent_prefill_tiles takes these (padded) sizes. */
+int latent_prefill_tiles_supported(int dim, int rot, int vdim) { return (dim == 64 || dim == 128) && rot == 64 && (vdim == 64 || vdim == 128); }
+
+/* ctx_rows: rows of ctx_kv and ctx_rot (all contexts). */
+int latent_prefill_tiles(const ncb_latent *g, long long ctx_rows, void *stream) {
+    if (!g) return NCB_ERR_ARG;
+    const int rc = check(*g);
+    if (rc != NCB_OK || g->n_tiles == 0) return rc;
+    if (!latent_prefill_tiles_supported(g->dim, g->rot, g->vdim) || !(g->scale > 0.f)) return NCB_ERR_UNSUPPORTED;
+    if (!g->ctx_kv || !g->ctx_rot || !g->out || !g->tile_row || !g->tile_rows || !g->tile_ctx || !g->tile_pos || g->n_tiles < 0 ||
+        g->n_tiles > 65535 || g->ctx_kv_ld < g->heads * (g->dim + g->vdim) || ctx_rows <= 0 || ctx_rows > 0x7fffffffLL || g->ldp > 0x7fffffffLL ||
+        g->off_q + (long long)g->heads * (g->dim + g->rot) > g->ldp)
+        return NCB_ERR_ARG;
+    if (g->ctx_kv_ld % 8 || g->ldo % 8 || ((uintptr_t)g->out | (uintptr_t)g->ctx_kv | (uintptr_t)g->ctx_rot) % 16) return NCB_ERR_ALIGN;
+    CUtensorMap q, kv, rot;
+    if (!tensor_map(g->proj, (int)g->rows, (int)g->ldp, att::ROWS, &q) || !tensor_map(g->ctx_kv, (int)ctx_rows, g->ctx_kv_ld, att::KEYS, &kv) ||
+        !tensor_map(g->ctx_rot, (int)ctx_rows, g->rot, att::KEYS, &rot))
+        return NCB_ERR_LAUNCH;
+    const dim3 grid(g->heads, g->n_tiles);
+    const cudaStream_t s = (cudaStream_t)stream;
+    auto run = [&](auto kernel, size_t smem) { return launch(kernel, grid, smem, att::THREADS, 1, s, q, kv, rot, *g); };
+    if (g->dim == 128)
+        return g->vdim == 128 ? run(k_latent_prefill_tiles<2, 3, 2>, att::Shape<3, 2, att::P_TWO, false>::SMEM_BYTES)
+                              : run(k_latent_prefill_tiles<2, 3, 1>, att::Shape<3, 1, att::P_TWO, false>::SMEM_BYTES);
+    return g->vdim == 128 ? run(k_latent_prefill_tiles<1, 2, 2>, att::Shape<2, 2, att::P_TWO, false>::SMEM_BYTES)
+                          : run(k_latent_prefill_tiles<1, 2, 1>, att::Shape<2, 1, att::P_TWO, false>::SMEM_BYTES);
 }
 
 } /* extern "C" */

@@ -227,9 +227,14 @@ class GroupedAttention:
         lib, bf = cuda_library("gqa_attn"), dtype == torch.bfloat16
         self.fused = bf and bool(lib.gqa_split_fused(self.dim, self.vdim))
         self.tiled = bf and bool(lib.gqa_prefill_supported(self.dim, self.vdim))
+        self.wide = self.tiled and self.scale > 0.0 and bool(lib.gqa_prefill_tiles_supported(self.dim, self.vdim))
 
     ROW_TILE = 64     # rows per tile of gqa_prefill
+    WIDE_TILE = 128   # rows per tile of gqa_prefill_tiles
     TILED_FROM = 8    # shorter segments run as rows on their own
+    # Segments from which gqa_prefill_tiles (tcgen05) has the pass. 10 heads of 128, us, gqa_prefill -> gqa_prefill_tiles: sixteen segments of
+    # 16 rows 11.3 -> 13.3, of 32 13.3 -> 13.3, of 100 21 -> 17; eight of 511 48 -> 28; one of 4,088 229 -> 105 (16 heads over 4: 335 -> 116).
+    WIDE_FROM = 32
 
     def new_cache(self, n_slots: int, max_len: int, of: "AttentionCache | None" = None) -> AttentionCache:
         if (of is None) != (self.kv_from is None):
@@ -286,9 +291,13 @@ class GroupedAttention:
         if out is not None:
             a.out, a.ldo = out.data_ptr(), out.stride(0)
         if out is not None and self.tiled and rows.plan is not None and rows.plan.longest >= self.TILED_FROM:
-            tiles, a.n_tiles = rows.plan.row_tiles(self.ROW_TILE)
+            wide = self.wide and rows.plan.longest >= self.WIDE_FROM
+            tiles, a.n_tiles = rows.plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
             a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
-            check(lib.gqa_prefill(pointer_to(a), stream()), "gqa_prefill")
+            if wide:
+                check(lib.gqa_prefill_tiles(pointer_to(a), stream()), "gqa_prefill_tiles")
+            else:
+                check(lib.gqa_prefill(pointer_to(a), stream()), "gqa_prefill")
         elif out is not None:
             max_len = min(rows.max_len, kv.capacity)
             tiles = (max_len + GQA_TILE - 1) // GQA_TILE
@@ -485,6 +494,8 @@ class LatentAttention:
         uv = pad_to(t["uv"].reshape(H, V, rank), H, self.vdim, self.rank)
         self.expanded = dtype == torch.bfloat16 and bool(
             cuda_library("latent_attn").latent_prefill_supported(self.dim, self.rot, self.vdim))
+        self.wide = self.expanded and self.scale > 0.0 and bool(
+            cuda_library("latent_attn").latent_prefill_tiles_supported(self.dim, self.rot, self.vdim))
         if self.expanded:  # both expansions of a latent row as one GEMM: per head the key's rows, then the value's
             both = torch.cat([uk, uv], 1).reshape(H * (self.dim + self.vdim), self.rank)
             self.w_ukv = pad_to(both, up(both.shape[0], 128), up(self.rank, 64)).to(dtype)
@@ -529,7 +540,11 @@ class LatentAttention:
             self._chunks[rows, max_len] = self.chunk_for([max_len] * rows, max_len)
         return self._chunks[rows, max_len]
 
-    ROW_TILE = 64  # rows per tile of latent_prefill
+    ROW_TILE = 64    # rows per tile of latent_prefill
+    WIDE_TILE = 128  # rows per tile of latent_prefill_tiles
+    # Segments from which latent_prefill_tiles (tcgen05) has the pass. 10 heads of 128 + 64 over 128, us, latent_prefill -> _tiles: sixteen
+    # segments of 16 rows 21.5 -> 21.5, of 100 42 -> 26; 16 rows behind 1,000 positions 60 -> 40; eight of 511 89 -> 46; one of 4,088 319 -> 126.
+    WIDE_FROM = 16
 
     def expands(self, plan: RowPlan) -> bool:
         """Whether a pass is cheaper with expanded keys and values: expanding every context once and attending in head
@@ -544,7 +559,8 @@ class LatentAttention:
     def run_expanded(self, a: Latent, rows: Rows) -> None:
         plan, lib, bf = rows.plan, cuda_library("latent_attn"), torch.bfloat16
         n_ctx = int((plan.starts + plan.count).sum())
-        (slots, first), (tiles, a.n_tiles) = plan.contexts(), plan.row_tiles(self.ROW_TILE)
+        wide = self.wide and plan.longest >= self.WIDE_FROM
+        (slots, first), (tiles, a.n_tiles) = plan.contexts(), plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
         N, K = self.w_ukv.shape
         a.rotate_q, a.max_len, a.n_contexts = 1, int((plan.starts + plan.count).max()), plan.n_segments
         a.ctx_slot, a.ctx_first = slots.data_ptr(), first.data_ptr()
@@ -558,7 +574,10 @@ class LatentAttention:
         g = GemmRs(x=a.ctx, w=self.w_ukv.data_ptr(), y=a.ctx_kv, rows=n_ctx, ldy=N, N=N, K=K, n_store=N, epilogue=0, scale=1.0,
                    status=a.status)
         check(cuda_library("tile_gemm").tile_gemm_rs(pointer_to(g), stream()), "tile_gemm_rs")
-        check(lib.latent_prefill(pointer_to(a), stream()), "latent_prefill")
+        if wide:
+            check(lib.latent_prefill_tiles(pointer_to(a), n_ctx, stream()), "latent_prefill_tiles")
+        else:
+            check(lib.latent_prefill(pointer_to(a), stream()), "latent_prefill")
 
     def run(self, proj: Tensor, cache: LatentCache, rows: Rows, out: "Tensor | None") -> None:
         n, f32, lib = rows.n, int(self.dtype == torch.float32), cuda_library("latent_attn")

@@ -144,6 +144,8 @@ SIGNATURES = {
         "latent_gather": ([c_ptr, c_ptr], c_int),
         "latent_prefill_supported": ([c_int] * 3, c_int),
         "latent_prefill": ([c_ptr, c_ptr], c_int),
+        "latent_prefill_tiles_supported": ([c_int] * 3, c_int),
+        "latent_prefill_tiles": ([c_ptr, c_ll, c_ptr], c_int),
     },
     "gla": {
         "gla_chunk_tokens": ([c_int], c_int),
@@ -158,6 +160,8 @@ SIGNATURES = {
         "gqa_split_fused": ([c_int] * 2, c_int),
         "gqa_prefill_supported": ([c_int] * 2, c_int),
         "gqa_prefill": ([c_ptr, c_ptr], c_int),
+        "gqa_prefill_tiles_supported": ([c_int] * 2, c_int),
+        "gqa_prefill_tiles": ([c_ptr, c_ptr], c_int),
     },
     "delta_rule": {
         "delta_step": ([c_ptr, c_int, c_ptr], c_int),

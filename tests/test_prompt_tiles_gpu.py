@@ -1,0 +1,110 @@
+"""Prompt attention on tcgen05 (csrc/attn_tiles.cuh) against float64 on the same operands and beside the kernels on mma.sync: runs of
+rows around the edges of a row tile (128) and a key tile (64), behind contexts of none, one and many keys, with NaN wherever the
+cache holds nothing. An output is one bf16 rounding (2^-9) of a sum whose weights carry 16 bits (11 over the fp8 cache)."""
+
+import ctypes
+
+import pytest
+import torch
+
+from nanochat_b200.mixers import RowPlan
+from nanochat_b200.native import Conv, Gqa, Latent, check, cuda_library, stream
+
+pytestmark = pytest.mark.gpu
+BF16, F64 = torch.bfloat16, torch.float64
+RUNS = [[(0, 1)], [(0, 64), (7, 63)], [(0, 65), (63, 130)], [(1, 127), (0, 128), (64, 129)], [(300, 257)], [(0, 700), (1000, 3), (5, 90)]]
+
+
+def attended(q, k, v, scale, start, sink=None):
+    """float64: q [n, H, D] at positions start .., k, v [H, start + n, ..] -> [n, H, V]; sink: logits of a key without a value."""
+    n, N = q.shape[0], k.shape[1]
+    s = torch.einsum("nhd,hkd->hnk", q.to(F64), k.to(F64)) * scale
+    seen = torch.arange(N, device=q.device)[None, :] <= torch.arange(start, start + n, device=q.device)[:, None]
+    s = s.masked_fill(~seen, float("-inf"))
+    if sink is not None:
+        s = torch.cat([s, sink.to(F64)[:, None, None].expand(-1, n, 1)], 2)
+    return torch.einsum("hnk,hkv->nhv", s.softmax(-1)[..., :N], v.to(F64))
+
+
+def off(got, want):
+    return float((got.to(F64) - want).norm() / want.norm())
+
+
+def judged(found, want):
+    """The new kernel within bf16's rounding of the value, and no further from it than the old one (rounding noise aside)."""
+    new, old = found
+    assert torch.isfinite(new.float()).all()
+    assert off(new, want) < 2 ** -8 and off(new, want) <= 1.05 * off(old, want) + 1e-6, (off(new, want), off(old, want))
+    assert float((new.to(F64) - want).abs().max()) <= 2 ** -7 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("runs", RUNS, ids=str)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 4, 128, 128), (6, 2, 128, 64), (4, 1, 64, 128), (2, 2, 64, 64)])
+def test_grouped(heads, kv_heads, dim, vdim, runs):
+    gen = torch.Generator(device="cuda").manual_seed(70)
+    slots, pos = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
+    n, capacity, scale = len(pos), 1088, 2.0 * dim ** -0.5
+    q = torch.randn(n, heads, dim, generator=gen, device="cuda").to(BF16)
+    kv = torch.full((len(runs), kv_heads, capacity, dim + vdim), float("nan"), dtype=BF16, device="cuda")
+    for s, (at, count) in enumerate(runs):
+        kv[s, :, :at + count] = torch.randn(kv_heads, at + count, dim + vdim, generator=gen, device="cuda").to(BF16)
+        kv[s, :, :at + count, :dim] *= (1 + (torch.arange(at + count, device="cuda") % 97 == 96))[None, :, None]  # maxima that move late
+    ldp = heads * dim  # the projection's rows: only the gate is read
+    proj = torch.randn(n, ldp, generator=gen, device="cuda").to(BF16)
+    dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slots)]
+    status, plan, lib, found = torch.zeros(1, dtype=torch.int32, device="cuda"), RowPlan(slots, pos, "cuda"), cuda_library("gqa_attn"), []
+    ring, taps = torch.zeros(len(runs), 1, ldp, dtype=BF16, device="cuda"), torch.ones(1, ldp, device="cuda")
+    for wide in (True, False):
+        out = torch.full((n, heads * vdim + 8), 7.0, dtype=BF16, device="cuda")
+        a = Gqa(conv=Conv(proj=proj.data_ptr(), ring=ring.data_ptr(), w=taps.data_ptr(), rows=n, ldp=ldp, taps=1, width=ldp, n_slots=len(runs),
+                          pos=dev[0].data_ptr(), slot_map=dev[1].data_ptr()), q=q.data_ptr(), kv=kv.data_ptr(), out=out.data_ptr(), ldo=out.stride(0),
+                heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, norm_count=dim, capacity=capacity, table_len=capacity, scale=scale, eps=1e-6,
+                status=status.data_ptr())
+        tiles, a.n_tiles = plan.row_tiles(128 if wide else 64)
+        a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+        check((lib.gqa_prefill_tiles if wide else lib.gqa_prefill)(ctypes.byref(a), stream()), "gqa")
+        assert int(status.item()) == 0 and bool((out[:, heads * vdim:] == 7.0).all())
+        found.append(out[:, :heads * vdim].view(n, heads, vdim))
+    want, row = [], 0
+    for s, (at, count) in enumerate(runs):
+        k, v = (t.repeat_interleave(heads // kv_heads, 0) for t in kv[s, :, :at + count].split([dim, vdim], -1))
+        want.append(attended(q[row:row + count], k, v, scale, at) * torch.sigmoid(proj[row:row + count, :heads].to(F64))[..., None])
+        row += count
+    judged(found, torch.cat(want))
+
+
+@pytest.mark.parametrize("runs", RUNS, ids=str)
+@pytest.mark.parametrize("heads,dim,vdim,sink,gated", [(3, 128, 128, True, True), (2, 128, 64, False, False), (2, 64, 128, True, False), (2, 64, 64, False, True)])
+def test_latent(heads, dim, vdim, sink, gated, runs):
+    gen, rot = torch.Generator(device="cuda").manual_seed(71), 64
+    slots, pos = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
+    n, contexts = len(pos), [at + count for at, count in runs]
+    ldp, ld, scale = heads * (dim + rot + vdim) + 8, heads * (dim + vdim) + 64, 2.0 * (dim + rot) ** -0.5
+    proj = torch.randn(n, ldp, generator=gen, device="cuda").to(BF16)
+    kv, kr = (torch.randn(sum(contexts), w, generator=gen, device="cuda").to(BF16) for w in (ld, rot))
+    sinks = torch.randn(heads, generator=gen, device="cuda")
+    dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slots)]
+    some = torch.ones(64, device="cuda")
+    status, plan, lib, found = torch.zeros(1, dtype=torch.int32, device="cuda"), RowPlan(slots, pos, "cuda"), cuda_library("latent_attn"), []
+    for wide in (True, False):
+        out = torch.full((n, heads * vdim + 8), 7.0, dtype=BF16, device="cuda")
+        a = Latent(proj=proj.data_ptr(), cache=kv.data_ptr(), out=out.data_ptr(), rows=n, ldp=ldp, ldo=out.stride(0), off_g=heads * (dim + rot), gated=int(gated),
+                   heads=heads, dim=dim, rot=rot, vdim=vdim, rank=32, norm_count=32, n_slots=len(runs), capacity=2000, table_len=2000, scale=scale,
+                   eps=1e-6, norm=some.data_ptr(), cos=some.data_ptr(), sin=some.data_ptr(), sink=sinks.data_ptr() if sink else None,
+                   pos=dev[0].data_ptr(), slot_map=dev[1].data_ptr(), ctx_rot=kr.data_ptr(), ctx_kv=kv.data_ptr(), ctx_kv_ld=ld, status=status.data_ptr())
+        tiles, a.n_tiles = plan.row_tiles(128 if wide else 64)
+        a.tile_row, a.tile_rows, a.tile_ctx, a.tile_pos = (t.data_ptr() for t in tiles)
+        check(lib.latent_prefill_tiles(ctypes.byref(a), sum(contexts), stream()) if wide else lib.latent_prefill(ctypes.byref(a), stream()), "latent")
+        assert int(status.item()) == 0 and bool((out[:, heads * vdim:] == 7.0).all())
+        found.append(out[:, :heads * vdim].view(n, heads, vdim))
+    want, row, first = [], 0, 0
+    for (at, count), length in zip(runs, contexts):
+        both = kv[first:first + length, :heads * (dim + vdim)].view(length, heads, dim + vdim).transpose(0, 1)
+        k = torch.cat([both[..., :dim], kr[first:first + length].expand(heads, -1, -1)], -1)
+        part = proj[row:row + count]
+        o = attended(part[:, :heads * (dim + rot)].view(count, heads, dim + rot), k, both[..., dim:], scale, at, sinks if sink else None)
+        if gated:
+            o = o * torch.sigmoid(part[:, heads * (dim + rot):heads * (dim + rot + vdim)].to(F64)).view(count, heads, vdim)
+        want.append(o)
+        row, first = row + count, first + length
+    judged(found, torch.cat(want))
