@@ -189,16 +189,71 @@ class PrefillPlan:
 
         slots, positions = np.asarray(slots, dtype=np.int32), np.asarray(positions, dtype=np.int32)
         self.rows_per_block = prefill_rows_per_block(Hq, cache.kv_heads)
-        starts = np.asarray(prefill_groups(slots, positions, self.rows_per_block), dtype=np.int32)
-        self.rows, self.n_groups = len(slots), len(starts) - 1
+        self.rows = n = len(slots)
+        start = np.ones(n, dtype=bool)  # a run: one slot, positions ascending by one
+        start[1:] = (slots[1:] != slots[:-1]) | (positions[1:] != positions[:-1] + 1)
+        first = np.flatnonzero(start).astype(np.int32)
+        count = np.diff(np.append(first, n)).astype(np.int32)
+        wide = self._wide_tiles(slots, positions, first, count, Hq, cache)
         # blocks start in list order: the groups that reach furthest into their prompts (most pages) go first, so
         # the short ones fill the gaps at the end
-        reach = positions[starts[1:] - 1] if self.n_groups else positions[:0]
-        order = np.argsort(-reach.astype(np.int64), kind="stable")
-        self.group_first = torch.from_numpy(starts[:-1][order].copy()).to(device)
-        self.group_rows = torch.from_numpy((starts[1:] - starts[:-1])[order].copy()).to(device)
-        self.slot_map = torch.from_numpy(slots).to(device)
-        self.lens = torch.from_numpy(positions + 1).to(device)
+        row, rows, pos = cut_runs(first, count, positions[first], self.rows_per_block)
+        order = np.argsort(-(pos + rows), kind="stable")
+        self.n_groups = len(row)
+        lists = [row[order], rows[order], slots, positions + 1, *(wide or [])]
+        flat = list(torch.from_numpy(np.concatenate(lists)).to(device).split([len(v) for v in lists]))  # one copy
+        self.group_first, self.group_rows, self.slot_map, self.lens = flat[:4]
+        self.wide = flat[4:] or None
+
+    # When prefill_attn_fp8_tiles (pages widened once, tcgen05) has the pass instead of prefill_attn_fp8, which widens a page for every
+    # block that reads it. Widening costs a launch and 50 KB of memory traffic per page and key/value head, so it pays where a page
+    # meets enough pairs (a row and a position it attends): with all query heads of a key/value head WIDE_GROUP_PAIRS or the widening
+    # of all pages small, and in any case WIDE_PAIRS. Measured, append and attention of whole prompts, heads over key/value heads, us,
+    # prefill_attn_fp8 -> tiles:
+    #   10 / 10   1 x 256  21.0 -> 16.5   8 x 256 31.6 -> 32.4   8 x 512 56.9 -> 55.8   16 x 100 24.8 -> 33.3    1 x 4096 243 -> 130
+    #   16 / 16   1 x 256  22.0 -> 18.8   8 x 256 39.6 -> 46.0   8 x 512 92.1 -> 80.7   16 x 100 34.9 -> 43.5    1 x 4096 337 -> 154
+    #   32 / 8    1 x 256  24.8 -> 17.9   8 x 256 56.0 -> 49.5   8 x 512 142 -> 98      16 x 100 39.9 -> 42.6    1 x 4096 625 -> 235
+    #   16 / 2    1 x 256  21.1 -> 15.1   8 x 256 30.3 -> 27.8   8 x 512 71.0 -> 50.2   16 x 100 21.2 -> 24.6    1 x 4096 317 -> 134
+    WIDE_ROWS = 64                # rows of a run, on average over the pass
+    WIDE_PAIRS = 6 * 1024         # per page and query head: about 96 positions a row
+    WIDE_GROUP_PAIRS = 12 * 1024  # per page and key/value head, or
+    WIDE_FEW = 128                # pages times key/value heads
+    WIDE_BYTES = 256 << 20        # of widened pages; passes that reach more run without them
+
+    def _wide_tiles(self, slots, positions, first, count, Hq: int, cache: Fp8KVCache) -> "list | None":
+        """The tile and page lists of prefill_attn_fp8_tiles for these runs, or None where prefill_attn_fp8 has the pass: short runs, more
+        pages than the workspace may take, and positions or slots outside the cache (which prefill_attn_fp8 flags)."""
+        import numpy as np
+
+        if self.rows < self.WIDE_ROWS * len(first) or not self.rows or not self.rows_per_block:
+            return None
+        ends = positions[first] + count  # positions of a run's context
+        pages = (ends + 63) // 64
+        total = int(pages.sum())
+        pairs = float((count * (ends - (count - 1) / 2)).sum())
+        few = total * cache.kv_heads <= self.WIDE_FEW
+        if pairs < self.WIDE_PAIRS * total or not (few or pairs * (Hq // cache.kv_heads) >= self.WIDE_GROUP_PAIRS * total):
+            return None
+        if slots.min() < 0 or slots.max() >= cache.n_slots or positions.min() < 0 or positions.max() >= cache.capacity:
+            return None
+        lib = cuda_library("prefill_attn")
+        row, rows, pos = cut_runs(first, count, positions[first], lib.prefill_attn_tile_rows())
+        if max(total, len(row)) > 65535 or lib.prefill_attn_tiles_bytes(cache.kv_heads, total) > self.WIDE_BYTES:
+            return None
+        page = (np.cumsum(pages) - pages)[np.searchsorted(first, row, side="right") - 1]
+        order = np.argsort(-pos, kind="stable")
+        index = np.arange(total) - np.repeat(np.cumsum(pages) - pages, pages)
+        lists = [v[order] for v in (row, rows, page, pos)] + [np.repeat(slots[first], pages), index, np.minimum(64, np.repeat(ends, pages) - 64 * index)]
+        return [v.astype(np.int32) for v in lists]
+
+
+def cut_runs(first, count, start, limit: int) -> tuple:
+    """Runs of rows (first row, rows, first position) cut into pieces of at most `limit` rows: the same three arrays."""
+    import numpy as np
+
+    per = (count + limit - 1) // limit
+    at = (np.arange(per.sum(), dtype=np.int32) - np.repeat(np.cumsum(per) - per, per).astype(np.int32)) * limit
+    return np.repeat(first, per) + at, np.minimum(limit, np.repeat(count, per) - at), np.repeat(start, per) + at
 
 
 def prefill_attention(q: Tensor, cache: Fp8KVCache, plan: PrefillPlan, softmax_scale: float | None = None,
@@ -212,6 +267,16 @@ def prefill_attention(q: Tensor, cache: Fp8KVCache, plan: PrefillPlan, softmax_s
     if out is None:
         out = torch.empty_like(q)
     scale = HEAD_DIM ** -0.5 if softmax_scale is None else softmax_scale
+    if plan.wide is not None:
+        row, count, page, pos, slots, index, used = plan.wide
+        lib = cuda_library("prefill_attn")
+        pages = torch.empty(lib.prefill_attn_tiles_bytes(cache.kv_heads, len(index)), dtype=torch.uint8, device=q.device)
+        rc = lib.prefill_attn_fp8_tiles(
+            pointer(q), pointer(cache.pages), pointer(row), pointer(count), pointer(page), pointer(pos), len(row), pointer(slots), pointer(index),
+            pointer(used), len(index), pointer(pages), pages.numel(), pointer(out), rows, Hq, cache.kv_heads, cache.pages_per_slot, scale,
+            pointer(status), stream())
+        check(rc, "prefill_attn_fp8_tiles")
+        return out
     rc = cuda_library("decode_attn").prefill_attn_fp8(
         pointer(q), pointer(cache.pages), pointer(plan.lens), pointer(plan.slot_map), pointer(plan.group_first),
         pointer(plan.group_rows), plan.n_groups, pointer(out), rows, Hq, cache.kv_heads, cache.n_slots, cache.pages_per_slot, scale,

@@ -23,7 +23,7 @@ INCLUDE = PACKAGE.parent / "include"
 NATIVE = PACKAGE / "_native"
 HEAD_DIM = 128
 LIBRARIES = ("kv_append", "decode_attn", "decode_step", "stream_gemm", "tile_gemm", "gemm_f32", "latent_attn", "gla",
-             "short_conv", "gqa_attn", "delta_rule")
+             "short_conv", "gqa_attn", "delta_rule", "prefill_attn")
 
 MAX_STREAMS = 8  # NCB_MAX_STREAMS
 c_ptr, c_int, c_ll, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
@@ -119,6 +119,11 @@ SIGNATURES = {
         "decode_attn_merge": ([c_ptr, c_int, c_ll, c_ptr, c_ptr], c_int),
         "decode_attn_fp8_sharded": ([c_ptr] * 5 + [c_ll, c_ptr] + [c_int] * 8 + [c_float, c_ptr, c_int, c_int, c_ptr,
                                                                                c_ptr, c_ptr], c_int),
+    },
+    "prefill_attn": {
+        "prefill_attn_tile_rows": ([], c_int),
+        "prefill_attn_tiles_bytes": ([c_int, c_int], c_ll),
+        "prefill_attn_fp8_tiles": ([c_ptr] * 6 + [c_int] + [c_ptr] * 3 + [c_int, c_ptr, c_ll, c_ptr, c_ll] + [c_int] * 3 + [c_float, c_ptr, c_ptr], c_int),
     },
     "decode_step": {
         "skinny_gemm": ([c_ptr] * 4 + [c_int] * 5 + [c_ptr], c_int),

@@ -7,6 +7,8 @@ import ctypes
 import pytest
 import torch
 
+import nanochat_b200 as ncb
+from nanochat_b200 import attention as ops
 from nanochat_b200.mixers import RowPlan
 from nanochat_b200.native import Conv, Gqa, Latent, check, cuda_library, stream
 
@@ -108,3 +110,55 @@ def test_latent(heads, dim, vdim, sink, gated, runs):
         want.append(o)
         row, first = row + count, first + length
     judged(found, torch.cat(want))
+
+
+@pytest.mark.parametrize("runs", RUNS, ids=str)
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (8, 2), (16, 1), (6, 2)])
+def test_fp8(Hq, Hkv, runs):
+    gen = torch.Generator(device="cuda").manual_seed(72)
+    lens = [at + n for at, n in runs]
+    cache = ncb.Fp8KVCache(len(runs), Hkv, max(lens) + 70)
+    kept = []
+    for s, n in enumerate(lens):
+        rows = [torch.randn(Hkv, cache.capacity, 128, generator=gen, device="cuda") * torch.rand(Hkv, cache.capacity, 1, generator=gen, device="cuda").mul_(4).exp2() for _ in "kv"]
+        rows[1][:, 1 + n // 2] = 0.0  # a value of zeros: its scale is zero
+        made = []
+        for t in rows:
+            scale = t.abs().amax(-1) / 448.0
+            b = (t / scale.clamp(min=1e-30)[..., None]).to(torch.float8_e4m3fn)
+            made.append((b.view(torch.uint8).clone(), scale, b.to(F64) * scale[..., None].to(F64)))
+            made[-1][0][:, n:], scale[:, n:] = 0x7f, float("nan")
+        cache.write(s, made[0][0], made[0][1], made[1][0], made[1][1])
+        kept.append([m[2][:, :n].repeat_interleave(Hq // Hkv, 0) for m in made])
+    slots, pos = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
+    q = torch.randn(len(pos), Hq, 128, generator=gen, device="cuda").to(BF16)
+    status, found = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    plan = ops.PrefillPlan.__new__(ops.PrefillPlan)
+    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
+    plan.__init__(slots, pos, Hq, cache, "cuda")
+    assert plan.wide is not None
+    for wide in (plan.wide, None):
+        plan.wide = wide
+        found.append(ops.prefill_attention(q, cache, plan, status=status))
+        assert int(status.item()) == 0
+    want, row = [], 0
+    for (at, n), (k, v) in zip(runs, kept):
+        want.append(attended(q[row:row + n], k, v, 128 ** -0.5, at))
+        row += n
+    judged(found, torch.cat(want))
+
+
+def test_fp8_route():
+    """Where the widened form does not apply the plan has none: short runs, a workspace beyond its bound, rows outside the cache."""
+    cache = ncb.Fp8KVCache(2, 2, 1024)
+    plan = lambda slots, pos, Hq=4: ops.PrefillPlan(slots, pos, Hq, cache, "cuda").wide  # noqa: E731
+    assert plan([0] * 700, list(range(700))) is not None and plan([0] * 200, list(range(200))) is not None
+    assert plan([0] * 150, list(range(150))) is None and plan([0] * 63, list(range(900, 963))) is None
+    assert plan([0] * 700, list(range(400, 1100))) is None and plan([2] * 700, list(range(700))) is None
+    assert plan([0] * 700, list(range(-1, 699))) is None
+    bound = ops.PrefillPlan.WIDE_BYTES
+    try:
+        ops.PrefillPlan.WIDE_BYTES = 1000
+        assert plan([0] * 700, list(range(700))) is None
+    finally:
+        ops.PrefillPlan.WIDE_BYTES = bound
