@@ -28,7 +28,7 @@
 namespace {
 
 constexpr int BM = 128;          /* rows per tile = MMA M */
-constexpr int THREADS = 192;     /* producer warp, MMA warp, four epilogue warps (eight for several streams: threads_of) */
+constexpr int THREADS = 192;     /* producer warp, MMA warp, four epilogue warps (eight where epilogue_warps says so: threads_of) */
 constexpr int A_BYTES = BM * KBLK * 2;
 
 constexpr int TURN_FLOATS = 32 * 33; /* per epilogue warp: see stream_columns */
@@ -36,8 +36,11 @@ constexpr int TURN_FLOATS = 32 * 33; /* per epilogue warp: see stream_columns */
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_RELU2 = 2, EPI_F32 = 3, EPI_GEGLU = 5, EPI_STREAM = 6, EPI_STREAMS = 7, EPI_SWIGLU = 8 };
 
 constexpr bool writes_stream(int epi) { return epi == EPI_STREAM || epi == EPI_STREAMS; }
-/* The update of several streams is bound by what its loads have in flight: twice as many warps share the columns of a tile. */
-__host__ __device__ constexpr int epilogue_warps(int epi) { return epi == EPI_STREAMS ? 8 : 4; }
+/* Epilogues that read something back (residual, streams: bound by what their loads have in flight) or compute much (silu) get twice as
+ * many warps, which share the columns of a tile. 4,088 rows x 1,280 (K 1,280 and 5,120 or 3,072 in turn), four -> eight warps, us: bf16
+ * residual 39.8 -> 38.6, stream 40.4 -> 34.5, two streams 37 -> 31; 6,144 wide: silu 78.6 -> 63.2. Plain stores, relu^2 and gelu gain
+ * nothing (41.3 -> 43.5, 48.2 -> 48.5, 60.3 -> 62.7). Loading the next columns' residual or stream ahead gains nothing on top. */
+__host__ __device__ constexpr int epilogue_warps(int epi) { return epi == EPI_RESID || epi == EPI_STREAM || epi == EPI_STREAMS || epi == EPI_SWIGLU ? 8 : 4; }
 constexpr int threads_of(int epi) { return THREADS + 32 * (epilogue_warps(epi) - 4); }
 constexpr int turn_bytes(int epi) { return writes_stream(epi) ? epilogue_warps(epi) * TURN_FLOATS * 4 : 0; }
 
