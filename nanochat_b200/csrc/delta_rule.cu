@@ -1147,6 +1147,7 @@ template <typename T> struct ConvLane {
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int back = 0; back < CONV_BATCH; back++) {
+            if (back >= a.conv.taps) continue; /* that row may be another sequence's: not even zero times its infinities */
             const float4 c = w[back], u = back ? old[CONV_BATCH - 1 - back] : x;
             y.x = fmaf(c.x, u.x, y.x), y.y = fmaf(c.y, u.y, y.y), y.z = fmaf(c.z, u.z, y.z), y.w = fmaf(c.w, u.w, y.w);
         }

@@ -43,3 +43,33 @@ def test_walk_equals_token_by_token(dtype, sizes):
     assert not out[idle].any() and torch.equal(last[1], want_last[1])
     assert float((last - want_last).abs().max() / want_last.abs().max()) < 1e-5
     assert float((out - want).abs().max() / want.abs().max()) < (2 ** -8 if dtype == torch.bfloat16 else 1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 6])
+def test_a_sequence_that_is_not_finite_stays_alone(dtype, taps):
+    """Sequences behind one that ends in infinities and NaN, from their start and behind a context: outputs and states bit for bit
+    those of a pass without it, whatever the taps (a tap that does not exist has no row, not one of weight zero)."""
+    entry, C = cases.delta(dim=32, vdim=32, heads=2, kv_heads=1, conv=taps), 64
+    state = cases.random_state(cases.config([entry], width=C), 64)
+    mixer = ChannelDelta(entry["mixer"], {k[7:]: v for k, v in state.items() if k.startswith("l0.mix.")}, 1e-5, 128, dtype, "cuda")
+    mixer.WALKED_FROM, mixer.CHUNKED_FROM = 2, 10 ** 9
+    runs = [(0, 0, 19), (1, 0, 9), (2, 5, 14)]  # slot, first position, rows
+    slots, pos = [s for s, _, n in runs for _ in range(n)], [p for _, at, n in runs for p in range(at, at + n)]
+    gen = torch.Generator(device="cuda").manual_seed(65)
+    proj = torch.randn(len(pos), mixer.in_width, generator=gen, device="cuda").to(dtype)
+    proj[16:19], proj[17] = float("inf"), float("nan")
+    found = []
+    for first in (0, 19):
+        cache, status = mixer.new_cache(3, 64), torch.zeros(1, dtype=torch.int32, device="cuda")
+        gen.manual_seed(66)
+        cache.state.state.normal_(generator=gen)
+        cache.ring.rows.copy_(torch.randn(cache.ring.rows.shape, generator=gen, device="cuda"))
+        part, n = proj[first:].contiguous(), len(pos) - first
+        out = torch.zeros((n, mixer.out_width), dtype=dtype, device="cuda")
+        mixer.run(part, cache, Rows(n, torch.tensor(pos[first:], dtype=torch.int32, device="cuda"), torch.tensor(slots[first:], dtype=torch.int32, device="cuda"), 64,
+                                    status, RowPlan(slots[first:], pos[first:], "cuda")), out)
+        assert int(status.item()) == 0
+        found.append((out[19 - first:], cache.state.state[1:]))
+    (out, last), (want, want_last) = found
+    assert bool(torch.isfinite(want.float()).all()) and torch.equal(out, want) and torch.equal(last, want_last)
