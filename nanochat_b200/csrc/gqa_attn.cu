@@ -167,6 +167,7 @@ template <typename T> __global__ void __launch_bounds__(THREADS, 7) k_gqa_rows(c
                 y[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int back = 0; back < CONV_BATCH; back++) {
+                    if (back >= a.conv.taps) continue; /* that row may be another sequence's: not even zero times its infinities */
                     const float4 c = f[back], u = v[OLD + e - back];
                     y[e].x = fmaf(c.x, u.x, y[e].x), y[e].y = fmaf(c.y, u.y, y[e].y), y[e].z = fmaf(c.z, u.z, y[e].z), y[e].w = fmaf(c.w, u.w, y[e].w);
                 }
@@ -232,6 +233,7 @@ template <typename T> __global__ void __launch_bounds__(THREADS, 7) k_gqa_rows(c
             } else {
 #pragma unroll
                 for (int back = 0; back < CONV_BATCH; back++) {
+                    if (back >= a.conv.taps) continue;
                     const float4 f = *reinterpret_cast<const float4 *>(w + back * size + i), v = load4(tile + (r + OLD - back) * size + i);
                     y.x = fmaf(f.x, v.x, y.x), y.y = fmaf(f.y, v.y, y.y), y.z = fmaf(f.z, v.z, y.z), y.w = fmaf(f.w, v.w, y.w);
                 }

@@ -150,6 +150,29 @@ def without(kv, position: int):
 
 
 @DTYPES
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("dim", [32, 160])
+def test_attention_rows_of_a_sequence_that_is_not_finite_stay_alone(dtype, dim, taps):
+    """The keys, values and outputs of a sequence that follows one with infinities and NaN in its last rows are those of the sequence
+    alone, bit for bit in the cache (the output's split into chunks depends on the pass)."""
+    entry, C = cases.attention(heads=2, kv_heads=1, dim=dim, vdim=32, conv=taps, rot_dims=16), 64
+    mixer = new_mixer(GroupedAttention, entry, cases.random_state(cases.config([entry], width=C), 57), dtype, 128)
+    slots, pos = [0] * 19 + [1] * 21, [*range(19), *range(21)]
+    proj = torch.randn(len(pos), mixer.in_width, generator=torch.Generator(device="cuda").manual_seed(58), device="cuda").to(dtype)
+    proj[16:19], proj[17] = float("inf"), float("nan")
+    found = []
+    for first in (0, 19):
+        cache, status = fresh_cache(mixer, 64), torch.zeros(1, dtype=torch.int32, device="cuda")
+        out = torch.zeros((len(pos) - first, mixer.out_width), dtype=dtype, device="cuda")
+        mixer.run(proj[first:].contiguous(), cache, rows_of(slots[first:], pos[first:], status), out)
+        assert int(status.item()) == 0
+        found.append((cache.kv.rows[1, :, :21].clone(), out[19 - first:]))
+    (kv, out), (want_kv, want) = found
+    assert bool(torch.isfinite(want_kv.float()).all()) and torch.equal(kv, want_kv)
+    close(out.cpu(), want.cpu(), dtype)
+
+
+@DTYPES
 def test_attention_over_another_layers_keys_and_values(dtype):
     first, second = cases.attention(), cases.attention(scale=0.9, kv_from=0)
     C, n = 64, 90
