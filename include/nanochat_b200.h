@@ -244,15 +244,15 @@ int prefill_attn_fp8(const void *q, const void *kv_cache, const void *lens, cons
  *   pages int32 [n_pages] each: slot, index in the slot, positions in use of every page of every sequence of the pass, a sequence's
  *   pages one after the other; tiles int32 [n_tiles] each: first row, rows (ascending positions of one sequence), the first page of
  *   the sequence in that list, the first row's position (row r of the tile attends positions [0, tile_pos + r]). List the tiles
- *   that reach furthest first. The caller has checked that slots and page indices are in the cache and that a sequence's pages
- *   cover its rows. Any Hq / Hkv. Two launches.
+ *   that reach furthest first. A page outside the cache (n_slots, pages_per_slot) is flagged NCB_DEV_BAD_LENGTH and not read: its
+ *   keys and values count as zeros. The caller has checked that a sequence's pages cover its rows. Any Hq / Hkv. Two launches.
  */
 int prefill_attn_tile_rows(void);
 long long prefill_attn_tiles_bytes(int Hkv, int n_pages);
 int prefill_attn_fp8_tiles(const void *q, const void *kv_cache, const void *tile_row, const void *tile_rows, const void *tile_page,
                            const void *tile_pos, int n_tiles, const void *page_slot, const void *page_index, const void *page_len,
                            int n_pages, void *workspace, long long workspace_bytes, void *out, long long rows, int Hq, int Hkv,
-                           int pages_per_slot, float softmax_scale, void *status, void *stream);
+                           int n_slots, int pages_per_slot, float softmax_scale, void *status, void *stream);
 
 /*
  * The first of decode_attn_fp8's two launches alone: the split-KV kernel, leaving one state per (b, h, chunk) in

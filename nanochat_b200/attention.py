@@ -204,6 +204,7 @@ class PrefillPlan:
         flat = list(torch.from_numpy(np.concatenate(lists)).to(device).split([len(v) for v in lists]))  # one copy
         self.group_first, self.group_rows, self.slot_map, self.lens = flat[:4]
         self.wide = flat[4:] or None
+        self.needs = (int(slots.max()) + 1, (int(positions.max()) + 64) // 64) if wide else (0, 0)  # slots and pages that `wide` lists
 
     # When prefill_attn_fp8_tiles (pages widened once, tcgen05) has the pass instead of prefill_attn_fp8, which widens a page for every
     # block that reads it. Widening costs a launch and 50 KB of memory traffic per page and key/value head, so it pays where a page
@@ -267,13 +268,15 @@ def prefill_attention(q: Tensor, cache: Fp8KVCache, plan: PrefillPlan, softmax_s
     if out is None:
         out = torch.empty_like(q)
     scale = HEAD_DIM ** -0.5 if softmax_scale is None else softmax_scale
-    if plan.wide is not None:
+    # a cache that lacks some of these (the plan was made for another one) goes to prefill_attn_fp8, which flags such rows
+    if plan.wide is not None and plan.needs[0] <= cache.n_slots and plan.needs[1] <= cache.pages_per_slot:
         row, count, page, pos, slots, index, used = plan.wide
         lib = cuda_library("prefill_attn")
         pages = torch.empty(lib.prefill_attn_tiles_bytes(cache.kv_heads, len(index)), dtype=torch.uint8, device=q.device)
         rc = lib.prefill_attn_fp8_tiles(
             pointer(q), pointer(cache.pages), pointer(row), pointer(count), pointer(page), pointer(pos), len(row), pointer(slots), pointer(index),
-            pointer(used), len(index), pointer(pages), pages.numel(), pointer(out), rows, Hq, cache.kv_heads, cache.pages_per_slot, scale,
+            pointer(used), len(index), pointer(pages), pages.numel(), pointer(out), rows, Hq, cache.kv_heads, cache.n_slots,
+            cache.pages_per_slot, scale,
             pointer(status), stream())
         check(rc, "prefill_attn_fp8_tiles")
         return out

@@ -38,15 +38,20 @@ struct WidenArgs {
     const int32_t *page_slot, *page_index, *page_len; /* of every page: its slot, its place there, positions in use */
     uint8_t *keys, *values;                           /* [Hkv][n_pages][WIDE_PAGE_BYTES] each */
     float *scales;                                    /* [Hkv][n_pages][3][64] */
-    int Hkv, pages_per_slot, n_pages;
+    int Hkv, n_slots, pages_per_slot, n_pages;
+    int *status;
 };
 
-/* Grid (Hkv, pages), 128 threads. Positions past the sequence's end become zeros: the cache holds anything there. */
+/* Grid (Hkv, pages), 128 threads. Positions past the sequence's end become zeros: the cache holds anything there; so does a page
+ * that is not in this cache (flagged: the lists may have been made for another one). */
 __global__ void __launch_bounds__(128) k_widen_pages(const WidenArgs a) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int kvh = blockIdx.x, p = blockIdx.y, tid = threadIdx.x, len = a.page_len[p];
-    const uint8_t *page = a.cache + (((size_t)a.page_slot[p] * a.Hkv + kvh) * a.pages_per_slot + a.page_index[p]) * PAGE_BYTES;
+    const int kvh = blockIdx.x, p = blockIdx.y, tid = threadIdx.x, slot = a.page_slot[p], index = a.page_index[p];
+    const bool ok = slot >= 0 && slot < a.n_slots && index >= 0 && index < a.pages_per_slot;
+    if (!ok && kvh == 0 && tid == 0) flag(a.status, NCB_DEV_BAD_LENGTH);
+    const int len = ok ? a.page_len[p] : 0;
+    const uint8_t *page = a.cache + (((size_t)(ok ? slot : 0) * a.Hkv + kvh) * a.pages_per_slot + (ok ? index : 0)) * PAGE_BYTES;
     const size_t to = (size_t)kvh * a.n_pages + p;
     uint4 *keys = reinterpret_cast<uint4 *>(a.keys + to * WIDE_PAGE_BYTES), *values = reinterpret_cast<uint4 *>(a.values + to * WIDE_PAGE_BYTES);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -135,9 +140,9 @@ long long prefill_attn_tiles_bytes(int Hkv, int n_pages) {
 
 int prefill_attn_fp8_tiles(const void *q, const void *kv_cache, const void *tile_row, const void *tile_rows, const void *tile_page,
                            const void *tile_pos, int n_tiles, const void *page_slot, const void *page_index, const void *page_len, int n_pages,
-                           void *workspace, long long workspace_bytes, void *out, long long rows, int Hq, int Hkv, int pages_per_slot,
+                           void *workspace, long long workspace_bytes, void *out, long long rows, int Hq, int Hkv, int n_slots, int pages_per_slot,
                            float softmax_scale, void *status, void *stream) {
-    if (rows < 0 || n_tiles < 0 || n_pages < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || pages_per_slot <= 0 || !(softmax_scale > 0.f)) return NCB_ERR_ARG;
+    if (rows < 0 || n_tiles < 0 || n_pages < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || n_slots <= 0 || pages_per_slot <= 0 || !(softmax_scale > 0.f)) return NCB_ERR_ARG;
     if (rows == 0 || n_tiles == 0) return NCB_OK;
     if (!q || !kv_cache || !tile_row || !tile_rows || !tile_page || !tile_pos || !page_slot || !page_index || !page_len || !workspace || !out ||
         n_pages == 0)
@@ -155,7 +160,7 @@ int prefill_attn_fp8_tiles(const void *q, const void *kv_cache, const void *tile
         !tensor_map(values, (int)pages * HEAD_DIM, PAGE_TOKENS, HEAD_DIM, &map_v))
         return NCB_ERR_LAUNCH;
     const WidenArgs wide = {(const uint8_t *)kv_cache, (const int32_t *)page_slot, (const int32_t *)page_index, (const int32_t *)page_len, keys, values,
-                            scales, Hkv, pages_per_slot, n_pages};
+                            scales, Hkv, n_slots, pages_per_slot, n_pages, (int *)status};
     const TilesArgs a = {(const int32_t *)tile_row, (const int32_t *)tile_rows, (const int32_t *)tile_page, (const int32_t *)tile_pos, scales,
                          (bf16 *)out, Hq, Hkv, n_pages, softmax_scale, (int *)status};
     cudaLaunchConfig_t config = {};

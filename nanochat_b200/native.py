@@ -123,7 +123,7 @@ SIGNATURES = {
     "prefill_attn": {
         "prefill_attn_tile_rows": ([], c_int),
         "prefill_attn_tiles_bytes": ([c_int, c_int], c_ll),
-        "prefill_attn_fp8_tiles": ([c_ptr] * 6 + [c_int] + [c_ptr] * 3 + [c_int, c_ptr, c_ll, c_ptr, c_ll] + [c_int] * 3 + [c_float, c_ptr, c_ptr], c_int),
+        "prefill_attn_fp8_tiles": ([c_ptr] * 6 + [c_int] + [c_ptr] * 3 + [c_int, c_ptr, c_ll, c_ptr, c_ll] + [c_int] * 4 + [c_float, c_ptr, c_ptr], c_int),
     },
     "decode_step": {
         "skinny_gemm": ([c_ptr] * 4 + [c_int] * 5 + [c_ptr], c_int),

@@ -14,6 +14,7 @@ from nanochat_b200.native import Conv, Gqa, Latent, check, cuda_library, stream
 
 pytestmark = pytest.mark.gpu
 BF16, F64 = torch.bfloat16, torch.float64
+NCB_DEV_BAD_LENGTH = 4
 RUNS = [[(0, 1)], [(0, 64), (7, 63)], [(0, 65), (63, 130)], [(1, 127), (0, 128), (64, 129)], [(300, 257)], [(0, 700), (1000, 3), (5, 90)]]
 
 
@@ -162,3 +163,40 @@ def test_fp8_route():
         assert plan([0] * 700, list(range(700))) is None
     finally:
         ops.PrefillPlan.WIDE_BYTES = bound
+
+
+def test_fp8_pages_outside_the_cache_are_flagged_and_not_read():
+    """A plan used with a cache of fewer slots, or of fewer pages: what lies outside is flagged and its rows are zero, as in a pass
+    that never had widened pages; the library on its own flags the pages, does not read them and takes zeros in their place."""
+    gen = torch.Generator(device="cuda").manual_seed(74)
+    large = ncb.Fp8KVCache(3, 2, 512)
+    raw = torch.randn(3, 2, 512, 128, generator=gen, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8)
+    ones = torch.ones(2, 512, device="cuda")
+    for s in range(3):
+        large.write(s, raw[s], ones, raw[s], ones)
+    for n_slots, capacity in ((1, 512), (2, 512), (3, 256), (2, 384)):
+        small = ncb.Fp8KVCache(n_slots, 2, capacity)
+        small.pages.copy_(large.pages[:n_slots, :, :small.pages_per_slot])
+        runs = [(0, 200), (1, 384), (2, 300)]
+        slots, pos = [s for s, n in runs for _ in range(n)], [p for _, n in runs for p in range(n)]
+        plan = ops.PrefillPlan(slots, pos, 4, large, "cuda")
+        assert plan.wide is not None
+        q = torch.randn(len(pos), 4, 128, generator=gen, device="cuda").to(BF16)
+        status, fine = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+        out, tiles = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
+        want = ops.prefill_attention(q, large, plan, status=fine)
+        ops.prefill_attention(q, small, plan, out=out, status=status)
+        assert int(fine.item()) == 0 and int(status.item()) == NCB_DEV_BAD_LENGTH
+        status.zero_()
+        plan.needs = (0, 0)  # past the check: the library's own
+        ops.prefill_attention(q, small, plan, out=tiles, status=status)
+        assert int(status.item()) == NCB_DEV_BAD_LENGTH and bool(torch.isfinite(tiles.float()).all())
+        row = 0
+        for s, n in runs:
+            if s < n_slots and n <= capacity:
+                assert off(out[row:row + n], want[row:row + n].double()) < 2 ** -7 and torch.equal(tiles[row:row + n], want[row:row + n])
+            elif s >= n_slots:
+                assert not out[row:row + n].any() and not tiles[row:row + n].any()
+            else:
+                assert not out[row + n - 22:row + n].any()  # at least the last block of rows
+            row += n
