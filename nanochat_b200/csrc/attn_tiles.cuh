@@ -70,16 +70,22 @@ __device__ __forceinline__ void umma_from_tmem(uint32_t tmem, uint32_t a, uint64
                  ::"r"(tmem), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
-/* 32 consecutive columns of this thread's lane, without waiting. */
-__device__ __forceinline__ void tmem_fetch32(uint32_t taddr, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+/* 64 consecutive columns of this thread's lane. One statement with its wait: nothing may use the registers in between. */
+__device__ __forceinline__ void tmem_fetch64(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 "
                  "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
+                 "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+                 "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                    "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-                   "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-                   "=r"(r[30]), "=r"(r[31])
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+                   "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+                   "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+                   "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+                   "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
                  : "r"(taddr)
                  : "memory");
 }
@@ -90,7 +96,6 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t *r) 
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_wait_load() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -227,9 +232,7 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
             fence_after();
             const int p0 = i * KEYS;
             uint32_t bits[KEYS];
-            tmem_fetch32(mine + (i & 1) * KEYS, bits);
-            tmem_fetch32(mine + (i & 1) * KEYS + 32, bits + 32);
-            tmem_wait_load();
+            tmem_fetch64(mine + (i & 1) * KEYS, bits);
             float s[KEYS];
 #pragma unroll
             for (int j = 0; j < KEYS; j++) s[j] = __uint_as_float(bits[j]);
@@ -272,13 +275,13 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                 m = grown ? best : m;
 #pragma unroll 1
                 for (int c = 0; c < VB * 2; c++) {
-                    uint32_t o[32];
-                    tmem_fetch32(o_mine + c * 32, o);
-                    tmem_wait_load();
+                    float o[32];
+                    tmem_load32(o_mine + c * 32, o);
+                    uint32_t u[32];
 #pragma unroll
-                    for (int j = 0; j < 32; j++) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-                    tmem_store16(o_mine + c * 32, o);
-                    tmem_store16(o_mine + c * 32 + 16, o + 16);
+                    for (int j = 0; j < 32; j++) u[j] = __float_as_uint(o[j] * f);
+                    tmem_store16(o_mine + c * 32, u);
+                    tmem_store16(o_mine + c * 32 + 16, u + 16);
                 }
             }
             float sum[2] = {0.f, 0.f};
@@ -326,10 +329,9 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
             fence_after();
 #pragma unroll 1
             for (int c = 0; c < VB * 2; c++) {
-                uint32_t o[32];
-                tmem_fetch32(o_mine + c * 32, o);
-                tmem_wait_load();
-                if (tid < w.rows) finish(tid, m, l, c * 32, reinterpret_cast<const float *>(o));
+                float o[32];
+                tmem_load32(o_mine + c * 32, o);
+                if (tid < w.rows) finish(tid, m, l, c * 32, o);
             }
         }
     }
