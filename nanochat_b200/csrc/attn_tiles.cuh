@@ -16,6 +16,9 @@
  * Measured (128 wide, two terms; 16 heads over 4, one prompt of 4,088 rows): 116 us = 592 TFLOP/s of causal pairs, the tensor pipe busy 60 %
  * of the cycles; the kernels on mma.sync, which re-read every key for each 16 rows as fragments, 335 us. Depth 192: 482 -> 140 us (165 with
  * two stages of keys and one of values: the next values' copy then stands between two products).
+ * A position that a row does not see must not reach it, not even as zero times a NaN or an infinity. Scores are masked; values are
+ * looked at in the two or three key tiles that the causal border crosses (each warp a quarter), and a tile that holds one that is
+ * not finite is multiplied by the softmax warps, row by row over the positions it sees, instead of by an MMA.
  * Every wait is bounded; when one expires NCB_DEV_WAIT_TIMEOUT is flagged and every role leaves its loop.
  */
 #pragma once
@@ -101,6 +104,22 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
+/* Whether some of the eight 16-bit values (IS_F16: f16, else bf16) is infinite or NaN: zero times it is not zero. */
+template <bool IS_F16> __device__ __forceinline__ bool not_finite8(uint4 v) {
+    uint32_t acc = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (IS_F16) asm("fma.rn.f16x2 %0, %1, %2, %0;" : "+r"(acc) : "r"((&v.x)[i]), "r"(0u));
+        else asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(acc) : "r"((&v.x)[i]), "r"(0u));
+    }
+    return (acc & 0x7fff7fffu) != 0;
+}
+/* Value column c of key j in a staged tile (both forms: 128-byte rows of eight 16-byte chunks, swizzled). */
+template <bool TRANSPOSED> __device__ __forceinline__ float staged_value(const uint8_t *tile, int j, int c) {
+    if (TRANSPOSED) return __half2float(*reinterpret_cast<const __half *>(tile + c * 128 + ((j / 8 ^ c & 7) * 16) + j % 8 * 2));
+    return __bfloat162float(*reinterpret_cast<const bf16 *>(tile + c / 64 * KEYS * 128 + j * 128 + ((c % 64 / 8 ^ j & 7) * 16) + c % 8 * 2));
+}
+
 /* The block's program. `work()` is called by every thread once the kernel before this one has finished; finish(row, m, l, c, v) gets
  * row `row` of the tile's O (un-normalised, relative to 2^m; l: the sum) 32 columns from c at a time. */
 template <int KB, int VB, int P, bool SCALED, typename GetWork, typename Finish>
@@ -110,13 +129,14 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
     const uint32_t base = smem_u32(raw), bars = base + S::AT_BARS;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(raw + S::AT_BARS + 128);
     volatile int *failed = reinterpret_cast<volatile int *>(raw + S::AT_BARS + 136);
-    /* k_full[2], v_full[2], s_full[2], p_ready[2], pv_done[2], q_full: the i-th key tile uses entry i % 2 of each (k_full: i % K_STAGES) */
+    volatile int *odd = failed + 1; /* per key tile that the causal border crosses (at most three): some value is not finite */
+    /* k_full[2], v_full[2], s_full[2], p_ready[2], pv_done[2], q_full, looked: the i-th key tile uses entry i % 2 of each (k_full: i % K_STAGES) */
     auto k_full = [&](int s) { return bars + 8u * s; };
     auto v_full = [&](int s) { return bars + 16u + 8u * s; };
     auto s_full = [&](int s) { return bars + 32u + 8u * s; };
     auto p_ready = [&](int s) { return bars + 48u + 8u * s; };
     auto pv_done = [&](int s) { return bars + 64u + 8u * s; };
-    const uint32_t q_full = bars + 80u;
+    const uint32_t q_full = bars + 80u, looked = bars + 88u;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < 2; s++) {
@@ -127,7 +147,8 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
             mbar_init(pv_done(s), 1);
         }
         mbar_init(q_full, 1);
-        *failed = 0;
+        mbar_init(looked, SOFTMAX_WARPS);
+        *failed = odd[0] = odd[1] = odd[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -143,6 +164,7 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const Work w = work();
     const int keys = w.pos0 + w.rows, n = w.rows > 0 ? (keys + KEYS - 1) / KEYS : 0;
+    const int border = (w.pos0 + 1) / KEYS; /* the first tile with a key that some row does not see */
     auto wait = [&](uint32_t bar, int use) { /* one thread */
         if (!*failed && mbar_wait(bar, use & 1)) return true;
         flag(status, NCB_DEV_WAIT_TIMEOUT);
@@ -212,11 +234,13 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                 if (!wait(v_full(i % S::V_STAGES), i / S::V_STAGES) || !wait(p_ready(i & 1), i >> 1)) break;
                 fence_after();
                 const uint32_t vs = base + S::AT_V + (i % S::V_STAGES) * S::V_BYTES, p = tmem + (i & 1) * KEYS;
+                if (i < border || !odd[i - border]) {
 #pragma unroll
-                for (int k = 0; k < KEYS / 16; k++) { /* 16 keys: 8 columns of packed probabilities */
-                    const uint64_t b = SCALED ? umma_desc(vs + k * 32) : desc_by_rows(vs + k * 2048, KEYS * 128);
-                    umma_from_tmem(t_out, p + k * 8, b, value, (i | k) != 0);
-                    if (P == P_TWO) umma_from_tmem(t_out, p + KEYS / 2 + k * 8, b, value, 1);
+                    for (int k = 0; k < KEYS / 16; k++) { /* 16 keys: 8 columns of packed probabilities */
+                        const uint64_t b = SCALED ? umma_desc(vs + k * 32) : desc_by_rows(vs + k * 2048, KEYS * 128);
+                        umma_from_tmem(t_out, p + k * 8, b, value, (i | k) != 0);
+                        if (P == P_TWO) umma_from_tmem(t_out, p + KEYS / 2 + k * 8, b, value, 1);
+                    }
                 }
                 umma_commit(pv_done(i & 1));
             }
@@ -284,6 +308,25 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                     tmem_store16(o_mine + c * 32 + 16, u + 16);
                 }
             }
+            if (i >= border) {
+                ok = wait_all(v_full(i % S::V_STAGES), i / S::V_STAGES);
+                if (!ok) break;
+                uint8_t *v = raw + S::AT_V + (i % S::V_STAGES) * S::V_BYTES;
+                const int used = SCALED ? KEYS : keys - p0; /* positions past the tile's last row may hold anything: zeros (SCALED: they are) */
+                bool strange = SCALED && tid < KEYS && !isfinite(reinterpret_cast<const float *>(sc)[2 * KEYS + tid]);
+#pragma unroll
+                for (int c = tid; c < VB * KEYS * 8; c += 32 * SOFTMAX_WARPS) {
+                    uint4 *chunk = reinterpret_cast<uint4 *>(v) + c;
+                    if (SCALED || c / 8 % KEYS < used) strange |= not_finite8<P == P_F16>(*chunk);
+                    else *chunk = make_uint4(0u, 0u, 0u, 0u);
+                }
+                if (!SCALED) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                strange = __any_sync(0xffffffffu, strange);
+                if (lane == 0) {
+                    if (strange) odd[i - border] = 1;
+                    arrive(looked);
+                }
+            }
             float sum[2] = {0.f, 0.f};
             const uint32_t p_mine = mine + (i & 1) * KEYS;
 #pragma unroll
@@ -309,16 +352,41 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                 if (P == P_TWO) tmem_store16(p_mine + KEYS / 2 + 16 * h, lo);
             }
             l += sum[0] + sum[1];
-            if (!SCALED && p0 + KEYS > keys) { /* positions past the tile's last row may hold anything, and 0 x NaN is NaN */
-                ok = wait_all(v_full(i % S::V_STAGES), i / S::V_STAGES);
+            if (i >= border) {
+                ok = wait_all(looked, i - border);
                 if (!ok) break;
-                const int first = keys - p0, count = KEYS - first; /* rows of every box */
-                uint8_t *v = raw + S::AT_V + (i % S::V_STAGES) * S::V_BYTES;
-                for (int c = tid; c < VB * count * 8; c += 32 * SOFTMAX_WARPS) {
-                    const int box = c / (count * 8), at = c % (count * 8);
-                    *reinterpret_cast<uint4 *>(v + box * KEYS * 128 + first * 128 + at * 16) = make_uint4(0u, 0u, 0u, 0u);
+                if (odd[i - border]) {
+                    const uint8_t *v = raw + S::AT_V + (i % S::V_STAGES) * S::V_BYTES;
+                    uint32_t u[KEYS];
+                    float p[KEYS]; /* the probabilities as the MMA would have read them */
+                    tmem_wait_store();
+                    tmem_fetch64(p_mine, u);
+#pragma unroll
+                    for (int j = 0; j < KEYS; j += 2) {
+                        const uint32_t hi = u[j / 2], lo = u[KEYS / 2 + j / 2];
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+                        p[j] = P == P_F16 ? f.x : __uint_as_float(hi << 16) + __uint_as_float(lo << 16);
+                        p[j + 1] = P == P_F16 ? f.y : __uint_as_float(hi & 0xffff0000u) + __uint_as_float(lo & 0xffff0000u);
+                    }
+                    ok = i == 0 || wait_all(pv_done((i - 1) & 1), (i - 1) >> 1); /* O is complete up to the tile before */
+                    if (!ok) break;
+                    fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < VB * 2; c++) {
+                        float o[32] = {};
+                        if (i > 0) tmem_load32(o_mine + c * 32, o);
+#pragma unroll 1
+                        for (int j = 0; j < KEYS && p0 + j <= last; j++)
+#pragma unroll
+                            for (int e = 0; e < 32; e++) o[e] = fmaf(p[j], staged_value<SCALED>(v, j, c * 32 + e), o[e]);
+                        __syncwarp();
+                        uint32_t u[32];
+#pragma unroll
+                        for (int e = 0; e < 32; e++) u[e] = __float_as_uint(o[e]);
+                        tmem_store16(o_mine + c * 32, u);
+                        tmem_store16(o_mine + c * 32 + 16, u + 16);
+                    }
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             tmem_wait_store();
             fence_before();

@@ -200,3 +200,83 @@ def test_fp8_pages_outside_the_cache_are_flagged_and_not_read():
             else:
                 assert not out[row + n - 22:row + n].any()  # at least the last block of rows
             row += n
+
+
+# (first position, rows) and where a value, key or scale is not finite: early, late and at the borders of a tile of the run
+PLANTED = [((0, 40), 5), ((0, 128), 127), ((0, 130), 64), ((63, 128), 100), ((62, 128), 130), ((200, 300), 430), ((200, 300), 201), ((7, 90), 96), ((0, 200), 0)]
+
+
+def split_at(got, clean, row, columns):
+    """Rows before `row` and all other columns as without the planted value, the rest not finite."""
+    rest = [c for c in range(clean.shape[-1]) if c not in columns]
+    assert torch.isfinite(got[:row].float()).all() and torch.isfinite(got[..., rest].float()).all()
+    assert row == 0 or off(got[:row], clean[:row]) < 2 ** -8
+    assert not rest or off(got[..., rest], clean[..., rest]) < 2 ** -8
+    assert not torch.isfinite(got[row:][..., columns].float()).any()
+
+
+@pytest.mark.parametrize("run,at", PLANTED, ids=str)
+@pytest.mark.parametrize("vdim,bad", [(64, float("nan")), (128, float("inf"))])
+def test_a_value_that_is_not_finite_reaches_only_rows_that_see_it(run, at, vdim, bad):
+    """Grouped and latent attention: one value of one position is infinite or NaN."""
+    gen, (start, n), heads, dim, rot = torch.Generator(device="cuda").manual_seed(75), run, 2, 128, 64
+    length, plan, status = start + n, RowPlan([0] * n, list(range(start, start + n)), "cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    pos, slots = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (range(start, start + n), [0] * n))
+    tiles, n_tiles = plan.row_tiles(128)
+    row, column = max(at - start, 0), 3
+    # grouped
+    q, kv = torch.randn(n, heads, dim, generator=gen, device="cuda").to(BF16), torch.randn(heads, 512, dim + vdim, generator=gen, device="cuda").to(BF16)
+    kv[:, length:] = float("nan")
+    clean = kv[:, :length].clone()
+    kv[:, at, dim + column] = bad
+    proj, ring, taps = torch.zeros(n, heads * dim, dtype=BF16, device="cuda"), torch.zeros(1, 1, heads * dim, dtype=BF16, device="cuda"), torch.ones(1, heads * dim, device="cuda")
+    out = torch.zeros((n, heads * vdim), dtype=BF16, device="cuda")
+    a = Gqa(conv=Conv(proj=proj.data_ptr(), ring=ring.data_ptr(), w=taps.data_ptr(), rows=n, ldp=heads * dim, taps=1, width=heads * dim, n_slots=1,
+                      pos=pos.data_ptr(), slot_map=slots.data_ptr()), q=q.data_ptr(), kv=kv.data_ptr(), out=out.data_ptr(), ldo=heads * vdim, heads=heads, kv_heads=heads,
+            dim=dim, vdim=vdim, norm_count=dim, capacity=512, table_len=512, scale=0.1, eps=1e-6, status=status.data_ptr(), n_tiles=n_tiles)
+    a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+    check(cuda_library("gqa_attn").gqa_prefill_tiles(ctypes.byref(a), stream()), "gqa_prefill_tiles")
+    assert int(status.item()) == 0
+    split_at(out.view(n, heads, vdim), 0.5 * attended(q, clean[..., :dim], clean[..., dim:], 0.1, start), row, [column])
+    # latent
+    width, ld = dim + rot, heads * (dim + vdim)
+    proj, ctx, kr = (torch.randn(m, w, generator=gen, device="cuda").to(BF16) for m, w in ((n, heads * width), (length, ld), (length, rot)))
+    both = ctx.view(length, heads, dim + vdim).transpose(0, 1).clone()
+    ctx.view(length, heads, dim + vdim)[at, :, dim + column] = bad
+    out, some = torch.zeros((n, heads * vdim), dtype=BF16, device="cuda"), torch.ones(64, device="cuda")
+    a = Latent(proj=proj.data_ptr(), cache=ctx.data_ptr(), out=out.data_ptr(), rows=n, ldp=heads * width, ldo=heads * vdim, heads=heads, dim=dim, rot=rot, vdim=vdim,
+               rank=32, norm_count=32, n_slots=1, capacity=512, table_len=512, scale=0.1, eps=1e-6, norm=some.data_ptr(), cos=some.data_ptr(), sin=some.data_ptr(),
+               pos=pos.data_ptr(), slot_map=slots.data_ptr(), ctx_rot=kr.data_ptr(), ctx_kv=ctx.data_ptr(), ctx_kv_ld=ld, status=status.data_ptr(), n_tiles=n_tiles)
+    a.tile_row, a.tile_rows, a.tile_ctx, a.tile_pos = (t.data_ptr() for t in tiles)
+    check(cuda_library("latent_attn").latent_prefill_tiles(ctypes.byref(a), length, stream()), "latent_prefill_tiles")
+    assert int(status.item()) == 0
+    want = attended(proj.view(n, heads, width), torch.cat([both[..., :dim], kr.expand(heads, -1, -1)], -1), both[..., dim:], 0.1, start)
+    split_at(out.view(n, heads, vdim), want, row, [column])
+
+
+@pytest.mark.parametrize("run,at", PLANTED, ids=str)
+@pytest.mark.parametrize("what", ["value", "value's scale", "key's scale"])
+def test_fp8_position_that_is_not_finite_reaches_only_rows_that_see_it(run, at, what):
+    gen, (start, n), Hkv = torch.Generator(device="cuda").manual_seed(76), run, 2
+    length = start + n
+    cache = ncb.Fp8KVCache(1, Hkv, 512)
+    raw = torch.randn(2, Hkv, 512, 128, generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    scale = torch.rand(2, Hkv, 512, generator=gen, device="cuda") + 0.5
+    k, v = (raw[i, :, :length].to(F64) * scale[i, :, :length, None].to(F64) for i in (0, 1))
+    b, columns, row = raw.view(torch.uint8).clone(), list(range(128)), max(at - start, 0)
+    b[:, :, length:], scale[:, :, length:] = 0x7f, float("nan")
+    if what == "value":
+        b[1, :, at, 3], columns = 0x7f, [3]
+    else:
+        scale[int(what[0] == "v"), :, at] = float("nan") if at % 2 else float("inf")
+    cache.write(0, b[0], scale[0], b[1], scale[1])
+    q = torch.randn(n, 4, 128, generator=gen, device="cuda").to(BF16)
+    status, plan = torch.zeros(1, dtype=torch.int32, device="cuda"), ops.PrefillPlan.__new__(ops.PrefillPlan)
+    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
+    plan.__init__([0] * n, list(range(start, length)), 4, cache, "cuda")
+    assert plan.wide is not None
+    got = ops.prefill_attention(q, cache, plan, softmax_scale=0.1, status=status)
+    assert int(status.item()) == 0
+    want = attended(q, k.repeat_interleave(2, 0), v.repeat_interleave(2, 0), 0.1, start)
+    rows = row if what == "key's scale" else n  # (rows that see such a key: NaN, or its value where it is the only one of weight)
+    split_at(got[:rows], want[:rows], row, columns)
