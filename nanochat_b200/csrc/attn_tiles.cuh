@@ -288,7 +288,7 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
             }
             const float best = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * (SCALED ? 1.f : w.scale);
             if (i == 0) {
-                m = best; /* finite: position 0 is seen by every row */
+                m = best; /* position 0 is seen by every row: finite, if its score is */
             } else if (__any_sync(0xffffffffu, best > m + RESCALE_LOG2)) {
                 const bool grown = best > m + RESCALE_LOG2;
                 const float f = grown ? ex2(m - best) : 1.f;
@@ -308,6 +308,12 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                     tmem_store16(o_mine + c * 32 + 16, u + 16);
                 }
             }
+            const bool none = SCALED && m == -INFINITY; /* no finite score so far: nothing counts yet, as in k_prefill_attn */
+            if (SCALED && __any_sync(0xffffffffu, none)) {
+#pragma unroll
+                for (int j = 0; j < KEYS; j++) s[j] = none ? -INFINITY : s[j];
+            }
+            const float reference = none ? 0.f : m;
             if (i >= border) {
                 ok = wait_all(v_full(i % S::V_STAGES), i / S::V_STAGES);
                 if (!ok) break;
@@ -335,7 +341,7 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
                     const int at = 32 * h + 2 * j;
-                    const float x = ex2(fmaf(s[at], w.scale, -m)), y = ex2(fmaf(s[at + 1], w.scale, -m));
+                    const float x = ex2(fmaf(s[at], w.scale, -reference)), y = ex2(fmaf(s[at + 1], w.scale, -reference));
                     sum[0] += x, sum[1] += y;
                     if (P == P_TWO) {
                         const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);

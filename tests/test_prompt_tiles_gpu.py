@@ -149,6 +149,29 @@ def test_fp8(Hq, Hkv, runs):
     judged(found, torch.cat(want))
 
 
+def test_fp8_rows_without_a_finite_score_are_zero():
+    """A query that is NaN, and a first position whose key is: nothing to attend, zeros, in both kernels."""
+    gen, n = torch.Generator(device="cuda").manual_seed(77), 200
+    cache = ncb.Fp8KVCache(1, 2, 256)
+    raw, scale = torch.randn(2, 256, 128, generator=gen, device="cuda").to(torch.float8_e4m3fn).view(torch.uint8), torch.ones(2, 256, device="cuda")
+    first = scale.clone()
+    first[1, 0] = float("nan")
+    cache.write(0, raw, first, raw, scale)
+    q = torch.randn(n, 4, 128, generator=gen, device="cuda").to(BF16)
+    q[70, 1] = float("nan")
+    status, found = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    plan = ops.PrefillPlan.__new__(ops.PrefillPlan)
+    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
+    plan.__init__([0] * n, list(range(n)), 4, cache, "cuda")
+    for wide in (plan.wide, None):
+        plan.wide = wide
+        found.append(ops.prefill_attention(q, cache, plan, status=status))
+        assert int(status.item()) == 0
+        assert not found[-1][70, 1].any() and not found[-1][0, 2:].any()
+        assert bool(torch.isfinite(found[-1][:, :2].float()).all()) and bool(torch.isnan(found[-1][1:, 2:].float()).all())
+    assert off(found[0][:, :2], found[1][:, :2].double()) < 2 ** -7
+
+
 def test_fp8_route():
     """Where the widened form does not apply the plan has none: short runs, a workspace beyond its bound, rows outside the cache."""
     cache = ncb.Fp8KVCache(2, 2, 1024)
