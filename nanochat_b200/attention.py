@@ -182,69 +182,99 @@ def prefill_rows_per_block(Hq: int, Hkv: int) -> int:
 class PrefillPlan:
     """What prefill_attention needs besides q for one pass of rows, built once per pass and shared by the layers: the
     row groups (longest first, so the blocks with the most pages start first), the rows' slots and lengths on the
-    device."""
+    device, and the tiles and pages of the rows that run on tcgen05.
 
-    def __init__(self, slots, positions, Hq: int, cache: Fp8KVCache, device):
+    spans: (first positions, ends) of the portions that the rows were given in, one of each per row, where a pass may hold part of a
+    portion only (default: the rows of the pass). Which kernel has a row follows from its portion and the cache's shape alone, and
+    neither kernel's sums for a row depend on its neighbours, so a row's bits depend neither on the other sequences of the pass nor
+    on where passes were cut. widen: True or False in place of the rule."""
+
+    def __init__(self, slots, positions, Hq: int, cache: Fp8KVCache, device, spans: "tuple | None" = None, widen: "bool | None" = None):
         import numpy as np
 
         slots, positions = np.asarray(slots, dtype=np.int32), np.asarray(positions, dtype=np.int32)
         self.rows_per_block = prefill_rows_per_block(Hq, cache.kv_heads)
         self.rows = n = len(slots)
-        start = np.ones(n, dtype=bool)  # a run: one slot, positions ascending by one
-        start[1:] = (slots[1:] != slots[:-1]) | (positions[1:] != positions[:-1] + 1)
-        first = np.flatnonzero(start).astype(np.int32)
-        count = np.diff(np.append(first, n)).astype(np.int32)
-        wide = self._wide_tiles(slots, positions, first, count, Hq, cache)
+        runs = np.asarray(prefill_groups(slots, positions, max(n, 1)))
+        first, count, pos = runs[:-1], np.diff(runs), positions[runs[:-1]].astype(np.int64)
+        begin, end = (pos, pos + count) if spans is None else (np.asarray(v, dtype=np.int64)[first] for v in spans)
+        wide = self._widened(slots[first], np.minimum(begin, pos), np.maximum(end, pos + count), Hq, cache, widen)
         # blocks start in list order: the groups that reach furthest into their prompts (most pages) go first, so
-        # the short ones fill the gaps at the end
-        row, rows, pos = cut_runs(first, count, positions[first], self.rows_per_block)
-        order = np.argsort(-(pos + rows), kind="stable")
-        self.n_groups = len(row)
-        lists = [row[order], rows[order], slots, positions + 1, *(wide or [])]
+        # the short ones fill the gaps at the end; all groups of prefill_attn_fp8's rows before those of the other rows
+        starts = np.asarray(prefill_groups(slots, positions, max(self.rows_per_block, 1)), dtype=np.int32)
+        row, rows = starts[:-1], np.diff(starts)
+        late = wide[np.searchsorted(first, row, side="right") - 1]
+        order = np.lexsort((-(positions[row].astype(np.int64) + rows), late))
+        self.n_groups, self.n_narrow = len(row), int(len(row) - late.sum())
+        batches = [self._tiles(*(v[part] for v in (slots[first], first, count, pos))) for part in self._batches(wide, pos + count, count, cache)]
+        lists = [row[order], rows[order], slots, positions + 1, *(v for batch in batches for v in batch)]
         flat = list(torch.from_numpy(np.concatenate(lists)).to(device).split([len(v) for v in lists]))  # one copy
         self.group_first, self.group_rows, self.slot_map, self.lens = flat[:4]
-        self.wide = flat[4:] or None
-        self.needs = (int(slots.max()) + 1, (int(positions.max()) + 64) // 64) if wide else (0, 0)  # slots and pages that `wide` lists
+        self.wide = [flat[i:i + 7] for i in range(4, len(flat), 7)] or None
+        # slots and pages that `wide` lists
+        self.needs = (int(slots[first][wide].max()) + 1, int((pos + count)[wide].max() + 63) // 64) if self.wide else (0, 0)
 
-    # When prefill_attn_fp8_tiles (pages widened once, tcgen05) has the pass instead of prefill_attn_fp8, which widens a page for every
+    # When prefill_attn_fp8_tiles (pages widened once, tcgen05) has a portion instead of prefill_attn_fp8, which widens a page for every
     # block that reads it. Widening costs a launch and 50 KB of memory traffic per page and key/value head, so it pays where a page
-    # meets enough pairs (a row and a position it attends): with all query heads of a key/value head WIDE_GROUP_PAIRS or the widening
-    # of all pages small, and in any case WIDE_PAIRS. Measured, append and attention of whole prompts, heads over key/value heads, us,
-    # prefill_attn_fp8 -> tiles:
+    # meets enough pairs (a row and a position it attends): WIDE_PAIRS, and with all query heads of a key/value head WIDE_GROUP_PAIRS.
+    # From position 0 that is 384 rows where every query head has its own key/value head, else 192. Measured, append and attention of
+    # whole prompts, heads over key/value heads, us, prefill_attn_fp8 -> tiles:
     #   10 / 10   1 x 256  21.0 -> 16.5   8 x 256 31.6 -> 32.4   8 x 512 56.9 -> 55.8   16 x 100 24.8 -> 33.3    1 x 4096 243 -> 130
     #   16 / 16   1 x 256  22.0 -> 18.8   8 x 256 39.6 -> 46.0   8 x 512 92.1 -> 80.7   16 x 100 34.9 -> 43.5    1 x 4096 337 -> 154
     #   32 / 8    1 x 256  24.8 -> 17.9   8 x 256 56.0 -> 49.5   8 x 512 142 -> 98      16 x 100 39.9 -> 42.6    1 x 4096 625 -> 235
     #   16 / 2    1 x 256  21.1 -> 15.1   8 x 256 30.3 -> 27.8   8 x 512 71.0 -> 50.2   16 x 100 21.2 -> 24.6    1 x 4096 317 -> 134
-    WIDE_ROWS = 64                # rows of a run, on average over the pass
+    # (A single prompt of 256 to 383 rows with equal heads would gain, eight of them would lose, and a row's kernel must not depend on
+    # the others.)
+    WIDE_ROWS = 64                # rows of a portion
     WIDE_PAIRS = 6 * 1024         # per page and query head: about 96 positions a row
-    WIDE_GROUP_PAIRS = 12 * 1024  # per page and key/value head, or
-    WIDE_FEW = 128                # pages times key/value heads
-    WIDE_BYTES = 256 << 20        # of widened pages; passes that reach more run without them
+    WIDE_GROUP_PAIRS = 12 * 1024  # per page and key/value head
+    WIDE_BYTES = 256 << 20        # of widened pages at a time; portions that reach more by themselves run without them
 
-    def _wide_tiles(self, slots, positions, first, count, Hq: int, cache: Fp8KVCache) -> "list | None":
-        """The tile and page lists of prefill_attn_fp8_tiles for these runs, or None where prefill_attn_fp8 has the pass: short runs, more
-        pages than the workspace may take, and positions or slots outside the cache (which prefill_attn_fp8 flags)."""
+    def _widened(self, slots, begin, end, Hq: int, cache: Fp8KVCache, widen: "bool | None"):
+        """Per run, from its portion [begin, end): whether prefill_attn_fp8_tiles has it. Never for heads that prefill_attn_fp8 refuses
+        and for rows outside the cache, which it flags."""
         import numpy as np
 
-        if self.rows < self.WIDE_ROWS * len(first) or not self.rows or not self.rows_per_block:
-            return None
-        ends = positions[first] + count  # positions of a run's context
+        count, pages = end - begin, (end + 63) // 64
+        pairs = count * (end - (count - 1) / 2)
+        rule = (count >= self.WIDE_ROWS) & (pairs >= self.WIDE_PAIRS * pages) & (pairs * (Hq // cache.kv_heads) >= self.WIDE_GROUP_PAIRS * pages)
+        able = (slots >= 0) & (slots < cache.n_slots) & (begin >= 0) & (end <= cache.capacity) & (self.rows_per_block > 0)
+        able &= (pages < 65536) & (pages * self._page_bytes(cache) <= self.WIDE_BYTES)
+        return able & (rule if widen is None else widen)
+
+    @staticmethod
+    def _page_bytes(cache: Fp8KVCache) -> int:
+        return cuda_library("prefill_attn").prefill_attn_tiles_bytes(cache.kv_heads, 1)
+
+    def _batches(self, wide, ends, count, cache: Fp8KVCache) -> list:
+        """The widened runs in groups that one call of prefill_attn_fp8_tiles takes: pages of WIDE_BYTES, 65,535 pages and tiles."""
+        import numpy as np
+
+        found, pages, tiles = [], 0, 0
+        most = min(self.WIDE_BYTES // self._page_bytes(cache), 65535)
+        for r in np.flatnonzero(wide).tolist():
+            p, t = (int(ends[r]) + 63) // 64, (int(count[r]) + 127) // 128
+            if not found or pages + p > most or tiles + t > 65535:
+                found.append([])
+                pages = tiles = 0
+            found[-1].append(r)
+            pages, tiles = pages + p, tiles + t
+        return found
+
+    @staticmethod
+    def _tiles(slots, first, count, pos) -> list:
+        """The tile lists (first row, rows, first page of the sequence, first position) and page lists (slot, index, positions in use)
+        of these runs; tiles that reach furthest first."""
+        import numpy as np
+
+        ends = pos + count
         pages = (ends + 63) // 64
-        total = int(pages.sum())
-        pairs = float((count * (ends - (count - 1) / 2)).sum())
-        few = total * cache.kv_heads <= self.WIDE_FEW
-        if pairs < self.WIDE_PAIRS * total or not (few or pairs * (Hq // cache.kv_heads) >= self.WIDE_GROUP_PAIRS * total):
-            return None
-        if slots.min() < 0 or slots.max() >= cache.n_slots or positions.min() < 0 or positions.max() >= cache.capacity:
-            return None
-        lib = cuda_library("prefill_attn")
-        row, rows, pos = cut_runs(first, count, positions[first], lib.prefill_attn_tile_rows())
-        if max(total, len(row)) > 65535 or lib.prefill_attn_tiles_bytes(cache.kv_heads, total) > self.WIDE_BYTES:
-            return None
-        page = (np.cumsum(pages) - pages)[np.searchsorted(first, row, side="right") - 1]
-        order = np.argsort(-pos, kind="stable")
-        index = np.arange(total) - np.repeat(np.cumsum(pages) - pages, pages)
-        lists = [v[order] for v in (row, rows, page, pos)] + [np.repeat(slots[first], pages), index, np.minimum(64, np.repeat(ends, pages) - 64 * index)]
+        base = np.cumsum(pages) - pages
+        row, rows, at = cut_runs(first, count, pos, cuda_library("prefill_attn").prefill_attn_tile_rows())
+        page = base[np.searchsorted(first, row, side="right") - 1]
+        order = np.argsort(-at, kind="stable")
+        index = np.arange(pages.sum()) - np.repeat(base, pages)
+        lists = [v[order] for v in (row, rows, page, at)] + [np.repeat(slots, pages), index, np.minimum(64, np.repeat(ends, pages) - 64 * index)]
         return [v.astype(np.int32) for v in lists]
 
 
@@ -268,22 +298,23 @@ def prefill_attention(q: Tensor, cache: Fp8KVCache, plan: PrefillPlan, softmax_s
     if out is None:
         out = torch.empty_like(q)
     scale = HEAD_DIM ** -0.5 if softmax_scale is None else softmax_scale
-    # a cache that lacks some of these (the plan was made for another one) goes to prefill_attn_fp8, which flags such rows
-    if plan.wide is not None and plan.needs[0] <= cache.n_slots and plan.needs[1] <= cache.pages_per_slot:
-        row, count, page, pos, slots, index, used = plan.wide
+    # a cache that lacks some of the listed pages (the plan was made for another one): prefill_attn_fp8 has all rows and flags those
+    fits = plan.wide is not None and plan.needs[0] <= cache.n_slots and plan.needs[1] <= cache.pages_per_slot
+    if fits:
         lib = cuda_library("prefill_attn")
-        pages = torch.empty(lib.prefill_attn_tiles_bytes(cache.kv_heads, len(index)), dtype=torch.uint8, device=q.device)
-        rc = lib.prefill_attn_fp8_tiles(
-            pointer(q), pointer(cache.pages), pointer(row), pointer(count), pointer(page), pointer(pos), len(row), pointer(slots), pointer(index),
-            pointer(used), len(index), pointer(pages), pages.numel(), pointer(out), rows, Hq, cache.kv_heads, cache.n_slots,
-            cache.pages_per_slot, scale,
-            pointer(status), stream())
-        check(rc, "prefill_attn_fp8_tiles")
-        return out
+        pages = torch.empty(lib.prefill_attn_tiles_bytes(cache.kv_heads, max(len(batch[5]) for batch in plan.wide)), dtype=torch.uint8, device=q.device)
+        for row, count, page, pos, slots, index, used in plan.wide:
+            rc = lib.prefill_attn_fp8_tiles(
+                pointer(q), pointer(cache.pages), pointer(row), pointer(count), pointer(page), pointer(pos), len(row), pointer(slots),
+                pointer(index), pointer(used), len(index), pointer(pages), pages.numel(), pointer(out), rows, Hq, cache.kv_heads, cache.n_slots,
+                cache.pages_per_slot, scale, pointer(status), stream())
+            check(rc, "prefill_attn_fp8_tiles")
+        if plan.n_narrow == 0:
+            return out
     rc = cuda_library("decode_attn").prefill_attn_fp8(
         pointer(q), pointer(cache.pages), pointer(plan.lens), pointer(plan.slot_map), pointer(plan.group_first),
-        pointer(plan.group_rows), plan.n_groups, pointer(out), rows, Hq, cache.kv_heads, cache.n_slots, cache.pages_per_slot, scale,
-        pointer(status), stream())
+        pointer(plan.group_rows), plan.n_narrow if fits else plan.n_groups, pointer(out), rows, Hq, cache.kv_heads, cache.n_slots,
+        cache.pages_per_slot, scale, pointer(status), stream())
     check(rc, "prefill_attn_fp8")
     return out
 

@@ -249,6 +249,7 @@ class StepDecoder:
         slot_rows = np.repeat(np.asarray(slots, dtype=np.int32), counts)
         pos_rows = np.concatenate([np.arange(n, dtype=np.int32) for n in counts])
         token_rows = np.concatenate([np.asarray(p[:-1], dtype=np.int64) for p in prompts])
+        spans = np.zeros(total, dtype=np.int32), np.repeat(np.asarray(counts, dtype=np.int32), counts)  # the prompt that a row is of
         for at in range(0, total, rows_per_pass):
             part = slice(at, min(at + rows_per_pass, total))
             n = part.stop - part.start
@@ -259,7 +260,8 @@ class StepDecoder:
             packed[n:].view(np.int32)[n:] = slot_rows[part]
             dev = torch.from_numpy(packed).to(self.device, non_blocking=True)
             tokens, small = dev[:n], dev[n:].view(torch.int32)
-            self.fill_rows(tokens, small[:n], small[n:], int(pos_rows[part].max()) + 1, (slot_rows[part], pos_rows[part]))
+            self.fill_rows(tokens, small[:n], small[n:], int(pos_rows[part].max()) + 1,
+                           (slot_rows[part], pos_rows[part], tuple(v[part] for v in spans)))
 
     @torch.no_grad()
     def feed(self, slot: int, tokens: list[int], start: int, want: list[int], rows_per_pass: int = 4096) -> Tensor:
@@ -291,7 +293,8 @@ class StepDecoder:
             dev = torch.tensor(tokens[at:at + m], dtype=torch.long).to(self.device)
             small = torch.from_numpy(np.concatenate([positions, slots])).to(self.device)
             places = [w - at for w in want if at <= w < at + m]
-            args = (dev, small[:m], small[m:], int(positions[-1]) + 1, (slots, positions))
+            spans = np.full(m, start, dtype=np.int32), np.full(m, start + n, dtype=np.int32)
+            args = (dev, small[:m], small[m:], int(positions[-1]) + 1, (slots, positions, spans))
             if places:
                 found.append(self.place_logits(*args, places))
             else:
@@ -472,7 +475,8 @@ class Decoder(StepDecoder):
         distinct_slots: no two rows share a slot (a decode step), so the attention kernel may append its own
         token; prefill passes, where rows of one sequence read each other's positions, need the separate append.
         host_rows: the rows' (slots, positions) as host lists, when the caller has them (prefill): attention then
-        runs in groups of consecutive rows that read a prompt's cache once per group instead of once per row."""
+        runs in groups of consecutive rows that read a prompt's cache once per group instead of once per row; a third
+        entry is PrefillPlan's spans."""
         cfg, lib, s = self.cfg, cuda_library("decode_step"), stream()
         rows, C = tokens.shape[0], cfg.hidden
         layers = self.w.layers
@@ -511,7 +515,7 @@ class Decoder(StepDecoder):
                 if i == cfg.n_layers - 1 and not attend_last_layer:
                     return h  # prefill: the last layer only has to fill its cache (decode.cu:862)
                 if grouped and plan is None:  # built while the GPU already runs the launches above
-                    plan = ops.PrefillPlan(host_rows[0], host_rows[1], cfg.n_heads, self.caches[0], self.device)
+                    plan = ops.PrefillPlan(host_rows[0], host_rows[1], cfg.n_heads, self.caches[0], self.device, *host_rows[2:])
                 if plan is not None:
                     att = ops.prefill_attention(q, self.caches[i], plan, out=att_buf, status=self.status)
                 else:

@@ -134,9 +134,7 @@ def test_fp8(Hq, Hkv, runs):
     slots, pos = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
     q = torch.randn(len(pos), Hq, 128, generator=gen, device="cuda").to(BF16)
     status, found = torch.zeros(1, dtype=torch.int32, device="cuda"), []
-    plan = ops.PrefillPlan.__new__(ops.PrefillPlan)
-    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
-    plan.__init__(slots, pos, Hq, cache, "cuda")
+    plan = ops.PrefillPlan(slots, pos, Hq, cache, "cuda", widen=True)  # the choice is not what is tested here
     assert plan.wide is not None
     for wide in (plan.wide, None):
         plan.wide = wide
@@ -160,9 +158,7 @@ def test_fp8_rows_without_a_finite_score_are_zero():
     q = torch.randn(n, 4, 128, generator=gen, device="cuda").to(BF16)
     q[70, 1] = float("nan")
     status, found = torch.zeros(1, dtype=torch.int32, device="cuda"), []
-    plan = ops.PrefillPlan.__new__(ops.PrefillPlan)
-    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
-    plan.__init__([0] * n, list(range(n)), 4, cache, "cuda")
+    plan = ops.PrefillPlan([0] * n, list(range(n)), 4, cache, "cuda", widen=True)
     for wide in (plan.wide, None):
         plan.wide = wide
         found.append(ops.prefill_attention(q, cache, plan, status=status))
@@ -202,8 +198,7 @@ def test_fp8_pages_outside_the_cache_are_flagged_and_not_read():
         small.pages.copy_(large.pages[:n_slots, :, :small.pages_per_slot])
         runs = [(0, 200), (1, 384), (2, 300)]
         slots, pos = [s for s, n in runs for _ in range(n)], [p for _, n in runs for p in range(n)]
-        plan = ops.PrefillPlan(slots, pos, 4, large, "cuda")
-        assert plan.wide is not None
+        plan = ops.PrefillPlan(slots, pos, 4, large, "cuda", widen=True)
         q = torch.randn(len(pos), 4, 128, generator=gen, device="cuda").to(BF16)
         status, fine = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
         out, tiles = torch.full_like(q, 7.0), torch.full_like(q, 7.0)
@@ -294,9 +289,7 @@ def test_fp8_position_that_is_not_finite_reaches_only_rows_that_see_it(run, at, 
         scale[int(what[0] == "v"), :, at] = float("nan") if at % 2 else float("inf")
     cache.write(0, b[0], scale[0], b[1], scale[1])
     q = torch.randn(n, 4, 128, generator=gen, device="cuda").to(BF16)
-    status, plan = torch.zeros(1, dtype=torch.int32, device="cuda"), ops.PrefillPlan.__new__(ops.PrefillPlan)
-    plan.WIDE_ROWS = plan.WIDE_PAIRS = plan.WIDE_GROUP_PAIRS = 0  # the choice is not what is tested here
-    plan.__init__([0] * n, list(range(start, length)), 4, cache, "cuda")
+    status, plan = torch.zeros(1, dtype=torch.int32, device="cuda"), ops.PrefillPlan([0] * n, list(range(start, length)), 4, cache, "cuda", widen=True)
     assert plan.wide is not None
     got = ops.prefill_attention(q, cache, plan, softmax_scale=0.1, status=status)
     assert int(status.item()) == 0

@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 V = 320
 
 
-def make(n_slots=4, store=0):
-    cfg = DecoderConfig(n_layers=2, hidden=512, n_heads=4, n_kv_heads=2, intermediate=1024, vocab=V, max_len=192)
+def make(n_slots=4, store=0, max_len=192, kv_heads=2):
+    cfg = DecoderConfig(n_layers=2, hidden=512, n_heads=4, n_kv_heads=kv_heads, intermediate=1024, vocab=V, max_len=max_len)
     w = DecoderWeights.random_init(cfg, seed=31, device="cuda", std=0.05)
     return NativeDecoder(Decoder(cfg, w, n_slots, prompt_store=store), end_token=V - 1)
 
@@ -50,6 +50,25 @@ def test_more_requests_than_slots_match_one_request_at_a_time():
     for i, r in enumerate(reqs):
         alone = dict(make(2).generate([r]))[0]
         assert alone == together[i], (i, alone, together[i])
+
+
+@pytest.mark.parametrize("kv_heads", [2, 4])
+def test_long_prompts_among_short_ones_match_each_alone(kv_heads):
+    """Prompts on both sides of the lengths from which prompt attention runs on other kernels, together and one at a time: the same
+    streams, and the same cache bytes however the passes are cut."""
+    prompts = [prompt(90 + i, n) for i, n in enumerate((301, 21, 701, 11, 151, 65, 500, 2))]
+    nd = make(3, max_len=1024, kv_heads=kv_heads)
+    reqs = [Request(input_ids=p, max_new_tokens=4) for p in prompts]
+    together = dict(nd.generate(reqs))
+    one = make(3, max_len=1024, kv_heads=kv_heads)
+    assert [dict(one.generate([r]))[0] for r in reqs] == [together[i] for i in range(len(reqs))]
+    want = make(8, max_len=1024, kv_heads=kv_heads).decoder
+    for b, p in enumerate(prompts):
+        want.prefill([p], [b])
+    for order, rows_per_pass in ((range(8), 4096), ([3, 7, 2, 5, 0, 1, 6, 4], 4096), (range(8), 512), ([6, 2, 1, 0, 5, 4, 3, 7], 330), (range(8), 100)):
+        got = make(8, max_len=1024, kv_heads=kv_heads).decoder
+        got.prefill([prompts[b] for b in order], list(order), rows_per_pass=rows_per_pass)
+        assert int(got.status.item()) == 0 and all(torch.equal(g.pages, w.pages) for g, w in zip(got.caches, want.caches))
 
 
 def test_stopping_criteria_token_limits_and_masks():

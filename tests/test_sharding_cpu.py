@@ -135,6 +135,67 @@ def test_prefill_groups_cut_runs_into_groups_that_share_page_loads():
     assert prefill_groups([3], [7], 2) == [0, 1]
 
 
+@pytest.mark.parametrize("heads", [(4, 4), (8, 2), (32, 1)])
+@pytest.mark.parametrize("pages_at_once", [8000, 40])
+def test_prompt_rows_take_their_kernel_by_their_own_portion(heads, pages_at_once, monkeypatch):
+    """PrefillPlan's lists on random passes, against a plain restatement: every row in one group or one tile, every tile's pages
+    listed, and the same rows widened whether their portion is alone, among others or cut into several passes."""
+    import random
+    from types import SimpleNamespace
+
+    from nanochat_b200 import attention as ops
+
+    (Hq, Hkv), rng = heads, random.Random(1)
+    cache, G = SimpleNamespace(kv_heads=Hkv, n_slots=5, capacity=4096), Hq // Hkv
+    monkeypatch.setattr(ops.PrefillPlan, "WIDE_BYTES", pages_at_once * ops.PrefillPlan._page_bytes(cache))
+
+    def by_rule(slot, begin, end):
+        pages, pairs = -(-end // 64), sum(range(begin + 1, end + 1))
+        rule = end - begin >= 64 and pairs >= 6144 * pages and pairs * G >= 12288 * pages
+        return rule and G <= 16 and pages <= pages_at_once and 0 <= slot < 5 and begin >= 0 and end <= 4096
+
+    def widened(plan, slots, positions):
+        """Rows in tiles, after checking the lists."""
+        groups = list(zip(plan.group_first.tolist(), plan.group_rows.tolist()))
+        assert len(groups) == plan.n_groups and sorted(r for f, n in groups for r in range(f, f + n)) == list(range(len(slots)))
+        for part in (groups[:plan.n_narrow], groups[plan.n_narrow:]):
+            reach = [positions[f + n - 1] for f, n in part]
+            assert reach == sorted(reach, reverse=True)
+        narrow, rows = {r for f, n in groups[:plan.n_narrow] for r in range(f, f + n)}, []
+        for batch in plan.wide or []:
+            row, count, page, pos, slot, index, used = (t.tolist() for t in batch)
+            assert len(slot) <= pages_at_once and pos == sorted(pos, reverse=True)
+            for f, n, p, at in zip(row, count, page, pos):
+                assert 0 < n <= 128 and positions[f:f + n] == list(range(at, at + n)) and len(set(slots[f:f + n])) == 1
+                for k in range(-(-(at + n) // 64)):
+                    assert slot[p + k] == slots[f] and index[p + k] == k and min(64, at + n - 64 * k) <= used[p + k] <= 64
+                rows += range(f, f + n)
+            assert plan.needs[0] > max(slot) and plan.needs[1] > max(index)
+        assert len(rows) == len(set(rows)) and narrow.isdisjoint(rows) and len(narrow) + len(rows) == len(slots)
+        return set(rows)
+
+    seen = 0
+    for _ in range(60):
+        portions = [(rng.choice([0, 1, 2, 3, 4, 4, 7]), rng.choice([0, 0, 0, -1, 30, 700, 3000]), rng.choice([1, 10, 63, 64, 150, 190, 200, 380, 390, 700, 1500]))
+                    for _ in range(rng.randint(1, 5))]
+        portions = [p for i, p in enumerate(portions) if p[0] not in [q[0] for q in portions[:i]]]
+        slots, positions = [s for s, _, n in portions for _ in range(n)], [p for _, at, n in portions for p in range(at, at + n)]
+        spans = [at for _, at, n in portions for _ in range(n)], [at + n for _, at, n in portions for _ in range(n)]
+        want = {r for r in range(len(slots)) if by_rule(slots[r], spans[0][r], spans[1][r])}
+        assert widened(ops.PrefillPlan(slots, positions, Hq, cache, "cpu"), slots, positions) == want
+        step, found = rng.choice([1, 7, 100, 333]), set()
+        for at in range(0, len(slots), step) if len(slots) < 300 * step else ():
+            part = slice(at, at + step)
+            plan = ops.PrefillPlan(slots[part], positions[part], Hq, cache, "cpu", tuple(v[part] for v in spans))
+            found |= {at + r for r in widened(plan, slots[part], positions[part])}
+        assert not found or found == want
+        seen += len(want)
+    assert (seen > 0) == (G <= 16)
+    assert ops.PrefillPlan([], [], Hq, cache, "cpu").n_groups == 0
+    forced = ops.PrefillPlan([1] * 3, [5, 6, 7], 4 * Hkv, cache, "cpu", widen=True)
+    assert widened(forced, [1] * 3, [5, 6, 7]) == {0, 1, 2} and ops.PrefillPlan([1] * 900, list(range(900)), 4 * Hkv, cache, "cpu", widen=False).wide is None
+
+
 def test_no_collection_restores_the_collector():
     import gc
 
