@@ -146,6 +146,12 @@ def padded_heads(w: Tensor, heads: int, size: int, padded: int) -> Tensor:
     return pad_to(w.reshape(heads, size, -1), heads, padded, w.shape[-1]).reshape(heads * padded, -1)
 
 
+def in_chunks(t: Tensor) -> bool:
+    """Whether rows of 16-bit values can be written 16 bytes at a time, as the tcgen05 prompt kernels do (the others take any even
+    stride)."""
+    return t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
 class ShortConv:
     """The short causal convolution on the first channels of a mixer's projection: fields [(channels x taps weights or None where
     there are none, the field's offset)]; channels outside the fields are zero."""
@@ -291,7 +297,7 @@ class GroupedAttention:
         if out is not None:
             a.out, a.ldo = out.data_ptr(), out.stride(0)
         if out is not None and self.tiled and rows.plan is not None and rows.plan.longest >= self.TILED_FROM:
-            wide = self.wide and rows.plan.longest >= self.WIDE_FROM
+            wide = self.wide and rows.plan.longest >= self.WIDE_FROM and in_chunks(out)
             tiles, a.n_tiles = rows.plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
             a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
             if wide:
@@ -371,7 +377,8 @@ class ChannelDelta:
             a.seg_first, a.seg_count, a.n_segments = first.data_ptr(), count.data_ptr(), plan.n_segments
         if plan is not None and self.chunk and plan.longest >= self.CHUNKED_FROM:
             self.run_chunked(a, rows)
-        elif plan is not None and self.walks and plan.longest >= self.WALKED_FROM:
+        elif (plan is not None and self.walks and plan.longest >= self.WALKED_FROM and proj.stride(0) % 8 == 0
+              and (out is None or out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0)):  # (what delta_step takes goes further)
             self.run_walk(a, rows)
         else:
             check(lib.delta_step(pointer_to(a), f32, stream()), "delta_step")
@@ -556,10 +563,10 @@ class LatentAttention:
         expanded = float(length.sum()) * self.rank * (self.dim + self.vdim) + pairs * (self.dim + self.rot + self.vdim)
         return expanded < 2.0 * pairs * (2 * self.rank + self.rot)
 
-    def run_expanded(self, a: Latent, rows: Rows) -> None:
+    def run_expanded(self, a: Latent, rows: Rows, out: Tensor) -> None:
         plan, lib, bf = rows.plan, cuda_library("latent_attn"), torch.bfloat16
         n_ctx = int((plan.starts + plan.count).sum())
-        wide = self.wide and plan.longest >= self.WIDE_FROM
+        wide = self.wide and plan.longest >= self.WIDE_FROM and in_chunks(out)
         (slots, first), (tiles, a.n_tiles) = plan.contexts(), plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
         N, K = self.w_ukv.shape
         a.rotate_q, a.max_len, a.n_contexts = 1, int((plan.starts + plan.count).max()), plan.n_segments
@@ -595,7 +602,7 @@ class LatentAttention:
         max_len = min(rows.max_len, cache.capacity)
         a.out, a.ldo = out.data_ptr(), out.stride(0)
         if rows.plan is not None and self.expands(rows.plan):
-            self.run_expanded(a, rows)
+            self.run_expanded(a, rows, out)
             return
         tiles = (max_len + LATENT_TILE - 1) // LATENT_TILE
         a.max_len, a.chunk_tiles = max_len, rows.chunk_tiles or self.default_chunk(n, max_len)

@@ -9,8 +9,9 @@ import torch
 
 import nanochat_b200 as ncb
 from nanochat_b200 import attention as ops
-from nanochat_b200.mixers import RowPlan
+from nanochat_b200.mixers import ChannelDelta, GroupedAttention, LatentAttention, RowPlan, Rows
 from nanochat_b200.native import Conv, Gqa, Latent, check, cuda_library, stream
+from tests import pudisun_cases, rekudra_cases
 
 pytestmark = pytest.mark.gpu
 BF16, F64 = torch.bfloat16, torch.float64
@@ -296,3 +297,41 @@ def test_fp8_position_that_is_not_finite_reaches_only_rows_that_see_it(run, at, 
     want = attended(q, k.repeat_interleave(2, 0), v.repeat_interleave(2, 0), 0.1, start)
     rows = row if what == "key's scale" else n  # (rows that see such a key: NaN, or its value where it is the only one of weight)
     split_at(got[:rows], want[:rows], row, columns)
+
+
+def mixer_of(kind: str):
+    """A mixer whose prompts run on tcgen05 (or as a walk), with random weights."""
+    if kind == "latent":
+        entry = pudisun_cases.latent(heads=2, dim=128, rot_dim=64, vdim=128)
+        state = pudisun_cases.random_state(pudisun_cases.config([entry], width=64), 81)
+    else:
+        entry = rekudra_cases.attention(heads=4, kv_heads=2, dim=128, vdim=128, rot_dims=32) if kind == "grouped" else rekudra_cases.delta(dim=64, vdim=64)
+        state = rekudra_cases.random_state(rekudra_cases.config([entry], width=64), 81)
+    cls = {"latent": LatentAttention, "grouped": GroupedAttention, "delta": ChannelDelta}[kind]
+    mixer = cls(entry["mixer"], {k[7:]: v for k, v in state.items() if k.startswith("l0.mix.")}, 1e-5, 128, BF16, "cuda")
+    mixer.expands = lambda plan: True
+    return mixer
+
+
+def run_counts(mixer, counts, proj, out=None):
+    """Segments of `counts` rows, each a slot of its own from position 0, through the mixer."""
+    slots, pos = [s for s, n in enumerate(counts) for _ in range(n)], [p for n in counts for p in range(n)]
+    status, n = torch.zeros(1, dtype=torch.int32, device="cuda"), len(pos)
+    out = torch.zeros((n, mixer.out_width), dtype=BF16, device="cuda") if out is None else out
+    dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slots)]
+    mixer.run(proj.clone(), mixer.new_cache(len(counts), 512), Rows(n, *dev, max(counts), status, RowPlan(slots, pos, "cuda")), out)
+    assert int(status.item()) == 0
+    return out
+
+
+@pytest.mark.parametrize("kind,off_by", [("latent", 2), ("grouped", 2), ("delta", 1), ("delta", 8)])
+def test_outputs_that_are_not_in_chunks_of_16_bytes(kind, off_by):
+    """Rows at a stride (or projections at one) that the kernels on tcgen05 and the walk do not take: the other kernels', bit for bit."""
+    mixer, counts = mixer_of(kind), [40, 17]
+    proj = torch.randn(sum(counts), mixer.in_width, generator=torch.Generator(device="cuda").manual_seed(82), device="cuda").to(BF16)
+    mixer.CHUNKED_FROM = 10 ** 9
+    out = torch.zeros((sum(counts), mixer.out_width + off_by), dtype=BF16, device="cuda")[:, :mixer.out_width]
+    found = run_counts(mixer, counts, proj, out)
+    if off_by % 8:
+        mixer.wide = mixer.walks = False
+    assert torch.equal(found, run_counts(mixer, counts, proj))
