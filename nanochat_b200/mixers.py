@@ -98,17 +98,27 @@ class RowPlan:
         out one after the other."""
         return self.upload("contexts", [self.slots, np.concatenate([[0], np.cumsum(self.starts + self.count)])])
 
-    def row_tiles(self, size: int) -> tuple[list[Tensor], int]:
+    def row_tiles(self, size: int, at_least: int = 1, below: int = 1 << 31) -> tuple[list[Tensor], int]:
         """([tile's first row, its rows, its context's first row, its first position], number of tiles) of at most `size`
-        rows of one segment, those that reach furthest into their sequences first."""
-        per = (self.count + size - 1) // size
+        rows of one segment, those that reach furthest into their sequences first; of the segments of at_least rows and more
+        that have fewer than `below`."""
+        some = np.flatnonzero((self.count >= at_least) & (self.count < below))
+        start, count, length = self.first[some], self.count[some], (self.starts + self.count)
+        per = (count + size - 1) // size
         within = np.arange(per.sum(), dtype=np.int32) - np.repeat(np.cumsum(per) - per, per)
-        first = np.repeat(self.first, per) + within * size
-        rows = np.minimum(size, np.repeat(self.first + self.count, per) - first)
-        context = np.repeat(np.cumsum(self.starts + self.count) - (self.starts + self.count), per)
-        pos = np.repeat(self.starts, per) + within * size
+        first = np.repeat(start, per) + within * size
+        rows = np.minimum(size, np.repeat(start + count, per) - first)
+        context = np.repeat((np.cumsum(length) - length)[some], per)
+        pos = np.repeat(self.starts[some], per) + within * size
         order = np.argsort(-pos.astype(np.int64), kind="stable")
-        return self.upload(("tiles", size), [v[order] for v in (first, rows, context, pos)]), len(first)
+        return self.upload(("tiles", size, at_least, below), [v[order] for v in (first, rows, context, pos)]), len(first)
+
+    def tile_lists(self, narrow: int, wide: int, wide_from: "int | None") -> list:
+        """row_tiles for two kernels, each by a segment's own rows: (True, lists, count) of the segments of wide_from rows and more in
+        tiles of `wide` (None: there are none), (False, lists, count) of the others in tiles of `narrow`; only what is not empty."""
+        if wide_from is None:
+            return [(False, *self.row_tiles(narrow))]
+        return [found for found in ((True, *self.row_tiles(wide, wide_from)), (False, *self.row_tiles(narrow, 1, wide_from))) if found[2]]
 
     def chunks(self, size: int) -> tuple[list[Tensor], int]:
         """([segment's first chunk (n + 1), chunk's first row, chunk's rows, the segment's rows before it], number of chunks) for
@@ -238,7 +248,7 @@ class GroupedAttention:
     ROW_TILE = 64     # rows per tile of gqa_prefill
     WIDE_TILE = 128   # rows per tile of gqa_prefill_tiles
     TILED_FROM = 8    # shorter segments run as rows on their own
-    # Segments from which gqa_prefill_tiles (tcgen05) has the pass. 10 heads of 128, us, gqa_prefill -> gqa_prefill_tiles: sixteen segments of
+    # Segments from which gqa_prefill_tiles (tcgen05) has them, beside shorter ones of the pass. 10 heads of 128, us, gqa_prefill -> gqa_prefill_tiles: sixteen segments of
     # 16 rows 11.3 -> 13.3, of 32 13.3 -> 13.3, of 100 21 -> 17; eight of 511 48 -> 28; one of 4,088 229 -> 105 (16 heads over 4: 335 -> 116).
     WIDE_FROM = 32
 
@@ -297,13 +307,10 @@ class GroupedAttention:
         if out is not None:
             a.out, a.ldo = out.data_ptr(), out.stride(0)
         if out is not None and self.tiled and rows.plan is not None and rows.plan.longest >= self.TILED_FROM:
-            wide = self.wide and rows.plan.longest >= self.WIDE_FROM and in_chunks(out)
-            tiles, a.n_tiles = rows.plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
-            a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
-            if wide:
-                check(lib.gqa_prefill_tiles(pointer_to(a), stream()), "gqa_prefill_tiles")
-            else:
-                check(lib.gqa_prefill(pointer_to(a), stream()), "gqa_prefill")
+            for wide, tiles, a.n_tiles in rows.plan.tile_lists(self.ROW_TILE, self.WIDE_TILE, self.WIDE_FROM if self.wide and in_chunks(out) else None):
+                a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+                entry = "gqa_prefill_tiles" if wide else "gqa_prefill"
+                check(getattr(lib, entry)(pointer_to(a), stream()), entry)
         elif out is not None:
             max_len = min(rows.max_len, kv.capacity)
             tiles = (max_len + GQA_TILE - 1) // GQA_TILE
@@ -549,7 +556,7 @@ class LatentAttention:
 
     ROW_TILE = 64    # rows per tile of latent_prefill
     WIDE_TILE = 128  # rows per tile of latent_prefill_tiles
-    # Segments from which latent_prefill_tiles (tcgen05) has the pass. 10 heads of 128 + 64 over 128, us, latent_prefill -> _tiles: sixteen
+    # Segments from which latent_prefill_tiles (tcgen05) has them, beside shorter ones of the pass. 10 heads of 128 + 64 over 128, us, latent_prefill -> _tiles: sixteen
     # segments of 16 rows 21.5 -> 21.5, of 100 42 -> 26; 16 rows behind 1,000 positions 60 -> 40; eight of 511 89 -> 46; one of 4,088 319 -> 126.
     WIDE_FROM = 16
 
@@ -566,12 +573,10 @@ class LatentAttention:
     def run_expanded(self, a: Latent, rows: Rows, out: Tensor) -> None:
         plan, lib, bf = rows.plan, cuda_library("latent_attn"), torch.bfloat16
         n_ctx = int((plan.starts + plan.count).sum())
-        wide = self.wide and plan.longest >= self.WIDE_FROM and in_chunks(out)
-        (slots, first), (tiles, a.n_tiles) = plan.contexts(), plan.row_tiles(self.WIDE_TILE if wide else self.ROW_TILE)
+        slots, first = plan.contexts()
         N, K = self.w_ukv.shape
         a.rotate_q, a.max_len, a.n_contexts = 1, int((plan.starts + plan.count).max()), plan.n_segments
         a.ctx_slot, a.ctx_first = slots.data_ptr(), first.data_ptr()
-        a.tile_row, a.tile_rows, a.tile_ctx, a.tile_pos = (t.data_ptr() for t in tiles)
         a.ctx_ld, a.ctx_kv_ld = K, N
         a.ctx = rows.buffer("latent_ctx", n_ctx * K, bf, self.device).data_ptr()
         a.ctx_rot = rows.buffer("latent_ctx_rot", n_ctx * self.rot, bf, self.device).data_ptr()
@@ -581,10 +586,12 @@ class LatentAttention:
         g = GemmRs(x=a.ctx, w=self.w_ukv.data_ptr(), y=a.ctx_kv, rows=n_ctx, ldy=N, N=N, K=K, n_store=N, epilogue=0, scale=1.0,
                    status=a.status)
         check(cuda_library("tile_gemm").tile_gemm_rs(pointer_to(g), stream()), "tile_gemm_rs")
-        if wide:
-            check(lib.latent_prefill_tiles(pointer_to(a), n_ctx, stream()), "latent_prefill_tiles")
-        else:
-            check(lib.latent_prefill(pointer_to(a), stream()), "latent_prefill")
+        for wide, tiles, a.n_tiles in plan.tile_lists(self.ROW_TILE, self.WIDE_TILE, self.WIDE_FROM if self.wide and in_chunks(out) else None):
+            a.tile_row, a.tile_rows, a.tile_ctx, a.tile_pos = (t.data_ptr() for t in tiles)
+            if wide:
+                check(lib.latent_prefill_tiles(pointer_to(a), n_ctx, stream()), "latent_prefill_tiles")
+            else:
+                check(lib.latent_prefill(pointer_to(a), stream()), "latent_prefill")
 
     def run(self, proj: Tensor, cache: LatentCache, rows: Rows, out: "Tensor | None") -> None:
         n, f32, lib = rows.n, int(self.dtype == torch.float32), cuda_library("latent_attn")

@@ -335,3 +335,14 @@ def test_outputs_that_are_not_in_chunks_of_16_bytes(kind, off_by):
     if off_by % 8:
         mixer.wide = mixer.walks = False
     assert torch.equal(found, run_counts(mixer, counts, proj))
+
+
+@pytest.mark.parametrize("kind", ["latent", "grouped"])
+def test_a_segments_length_chooses_its_kernel(kind):
+    """Long and short segments in one pass: every one as in a pass of its own, bit for bit."""
+    mixer, counts = mixer_of(kind), [200, 10, 40, 15, 31, 16, 32, 130, 8]
+    proj = torch.randn(sum(counts), mixer.in_width, generator=torch.Generator(device="cuda").manual_seed(83), device="cuda").to(BF16)
+    together, row = run_counts(mixer, counts, proj), 0
+    for n in counts:
+        assert torch.equal(together[row:row + n], run_counts(mixer, [n], proj[row:row + n])), n
+        row += n
