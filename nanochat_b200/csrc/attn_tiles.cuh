@@ -29,6 +29,9 @@ namespace {
 namespace att {
 
 constexpr int ROWS = 128, KEYS = 64, THREADS = 192, SOFTMAX_WARPS = 4;
+/* What the kernels declare instead of THREADS: two blocks of it leave a thread 128 registers. Two blocks of 192 threads would leave
+ * 168, but a block's warps 0, 1, 4 and 5 share two of the SM's four schedulers, whose registers then hold one block only. */
+constexpr int BOUND = 256;
 constexpr float RESCALE_LOG2 = 7.f; /* growth of a row's maximum that O may lag behind, in powers of two */
 constexpr float LOG2_E = 1.4426950408889634f;
 

@@ -717,7 +717,7 @@ template <int QS, int VN, bool EXACT> __global__ void __launch_bounds__(THREADS,
 
 /* Grid (heads, row tiles): the same for at most att::ROWS rows per tile on tcgen05 (attn_tiles.cuh); dim = 64 KB, vdim = 64 VB. Queries
  * and the cache are read as matrices of heads * dim and dim + vdim columns. */
-template <int KB, int VB> __global__ void __launch_bounds__(att::THREADS, 2) k_gqa_prefill_tiles(const __grid_constant__ CUtensorMap map_q,
+template <int KB, int VB> __global__ void __launch_bounds__(att::BOUND, 2) k_gqa_prefill_tiles(const __grid_constant__ CUtensorMap map_q,
                                                                                              const __grid_constant__ CUtensorMap map_kv, const ncb_gqa a) {
     extern __shared__ __align__(128) uint8_t raw[];
     const int h = blockIdx.x, tile = blockIdx.y;

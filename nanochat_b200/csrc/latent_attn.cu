@@ -798,7 +798,7 @@ template <int QS, int VN, bool EXACT> __global__ void __launch_bounds__(THREADS,
 
 /* Grid (heads, row tiles): the same for at most att::ROWS rows per tile on tcgen05 (attn_tiles.cuh); dim = 64 KA, dim + rot = 64 KB,
  * vdim = 64 VB. The projection, the expanded keys and values and the rotated parts are read as matrices. */
-template <int KA, int KB, int VB> __global__ void __launch_bounds__(att::THREADS, 2)
+template <int KA, int KB, int VB> __global__ void __launch_bounds__(att::BOUND, 2)
 k_latent_prefill_tiles(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_rot,
                        const ncb_latent a) {
     extern __shared__ __align__(128) uint8_t raw[];

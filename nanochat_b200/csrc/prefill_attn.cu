@@ -107,7 +107,7 @@ struct TilesArgs {
 
 /* Grid (Hq, tiles): see attn_tiles.cuh. A probability times 256 and the value's scale is at most 2^15 in f16: as many bits as in
  * k_prefill_attn. */
-__global__ void __launch_bounds__(att::THREADS, 2) k_prefill_tiles(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+__global__ void __launch_bounds__(att::BOUND, 2) k_prefill_tiles(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                                                    const __grid_constant__ CUtensorMap map_v, const TilesArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int h = blockIdx.x, tile = blockIdx.y;
