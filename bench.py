@@ -914,7 +914,7 @@ def bench_hybrid_kernels(device, profiled: bool = False) -> dict:
         seen = spy("latent_attn", lambda: latent.run(proj, cache, rows, mixed), ("latent_append", "latent_gather", "latent_prefill_tiles"))
         flops = prompts * n * (n + 1) // 2 * H * 2 * (192 + 128)
         us = per_call(lambda i: lib.latent_prefill_tiles(ctypes.byref(seen["latent_prefill_tiles"]), n * prompts, stream()), 20)
-        out[f"{name} latent_prefill"] = {"us": us, "flops": flops, "tflops": flops / us / 1e6, "frac_tensor": flops / us / 1e6 / tensor}
+        out[f"{name} latent_prefill_tiles"] = {"us": us, "flops": flops, "tflops": flops / us / 1e6, "frac_tensor": flops / us / 1e6 / tensor}
         us = per_call(lambda i: lib.latent_append(ctypes.byref(seen["latent_append"]), 0, stream()), 20)
         nbytes = n * prompts * 2 * (2 * 576 + 2 * H * 64)
         out[f"{name} latent_append"] = {"us": us, "bytes": nbytes, "gbs": nbytes / us / 1e3, "frac_hbm": nbytes / us / 1e3 / hbm}
@@ -1062,7 +1062,7 @@ def bench_rekudra_kernels(device, profiled: bool = False) -> dict:
             mixed = torch.empty(n * prompts, attn.out_width, dtype=torch.bfloat16, device=device)
             seen = spy("gqa_attn", lambda: attn.run(proj, cache, rows, mixed), ("gqa_rows", "gqa_prefill_tiles"))
             us = per_call(lambda i: lib.gqa_prefill_tiles(ctypes.byref(seen["gqa_prefill_tiles"]), stream()), 20)
-            multiplied(f"{name} gqa_prefill{label}", us, prompts * n * (n + 1) // 2 * H * 2 * 256)
+            multiplied(f"{name} gqa_prefill_tiles{label}", us, prompts * n * (n + 1) // 2 * H * 2 * 256)
             us = per_call(lambda i: lib.gqa_rows(ctypes.byref(seen["gqa_rows"]), 0, stream()), 20)
             moved(f"{name} gqa_rows{label}", us, 2 * 2 * n * prompts * (H * 128 + G * 256))
             state = delta.new_cache(prompts, 64)

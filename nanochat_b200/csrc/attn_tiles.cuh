@@ -7,7 +7,8 @@
  * columns) let the next tile's scores run under this tile's softmax; with O (at most 128 columns) a block takes 256 columns and at
  * most 113 KB of shared memory, so TWO blocks share an SM and one's MMAs run under the other's exponentials.
  *   - warps 0..3: softmax. O is rescaled only when a row's maximum has grown by more than 2^7 since the last time (the
- *     sum and O share the reference, so this is exact; a probability is at most 128);
+ *     sum and O share the reference, so this is exact; a probability, SCALED its product with the value's scale, is at most
+ *     128, and the sum of SCALED probabilities, whose reference counts a scale of 2^-64 at least, stays below 2^90);
  *   - warp 4, one thread: TMA boxes of 64 columns (128-byte swizzle), V two stages, K two where they fit, else one;
  *   - warp 5, one thread: MMAs.
  * A probability enters the second product as two bf16 terms (hi + lo, 16 bits; P_TWO) or as one f16 (P_F16). The tensor cores
@@ -19,7 +20,7 @@
  * A position that a row does not see must not reach it, not even as zero times a NaN or an infinity. Scores are masked; values are
  * looked at in the two or three key tiles that the causal border crosses (each warp a quarter), and a tile that holds one that is
  * not finite is multiplied by the softmax warps, row by row over the positions it sees, instead of by an MMA.
- * Every wait is bounded; when one expires NCB_DEV_WAIT_TIMEOUT is flagged and every role leaves its loop.
+ * Every wait on a barrier is bounded; when one expires NCB_DEV_WAIT_TIMEOUT is flagged and every role leaves its loop.
  */
 #pragma once
 

@@ -1,5 +1,5 @@
 /*
- * Shared by kv_append.cu and decode_attn.cu: the page layout of the fp8 KV cache (described in
+ * Shared by the libraries: the page layout of the fp8 KV cache (described in
  * include/nanochat_b200.h), status codes and small device helpers.
  */
 #pragma once
@@ -45,6 +45,14 @@ static __device__ __forceinline__ float ex2(float x) { /* exp2, -inf -> 0 */
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+/* The four e4m3 bytes of x as two f16x2 words (exact): lo from bytes 0, 1, hi from bytes 2, 3. */
+static __device__ __forceinline__ void widen_e4m3x4(uint32_t x, uint32_t &lo, uint32_t &hi) {
+    uint16_t l, h;
+    asm("mov.b32 {%0, %1}, %2;" : "=h"(l), "=h"(h) : "r"(x));
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(lo) : "h"(l));
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(hi) : "h"(h));
 }
 
 /* Where a sequence's attended positions and pages lie; shared by the split kernel and everything that merges its states. */

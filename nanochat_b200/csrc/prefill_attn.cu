@@ -20,13 +20,6 @@ __device__ __forceinline__ float lg2(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-/* The four e4m3 bytes of x as two f16x2 words (exact): lo from bytes 0, 1, hi from bytes 2, 3. */
-__device__ __forceinline__ void widen_e4m3x4(uint32_t x, uint32_t &lo, uint32_t &hi) {
-    uint16_t l, h;
-    asm("mov.b32 {%0, %1}, %2;" : "=h"(l), "=h"(h) : "r"(x));
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(lo) : "h"(l));
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(hi) : "h"(h));
-}
 
 /* A page widened to 16 bits, both exact: keys bf16 [64][128] (the queries' type), values f16 transposed [128][64] (the probabilities'),
  * and per position the key's scale, log2 of the value's scale, and that scale times P_SCALE. Every key/value head's pages follow

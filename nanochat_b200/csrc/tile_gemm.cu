@@ -392,7 +392,7 @@ constexpr bool PAIR_BY_DEFAULT = true;
  *   - MMA thread (leader only): waits for a full stage, issues the four K = 16 steps, and releases the stage in both
  *     blocks with one tcgen05.commit addressed to both blocks of the pair; the same for a finished accumulator;
  *   - epilogue warps (both blocks): as in the single-block kernel on the block's own 128 rows; every warp of both blocks
- *     then arrives on the leader's "accumulator drained" barrier (eight arrivals).
+ *     then arrives on the leader's "accumulator drained" barrier (eight arrivals, sixteen with eight epilogue warps per block).
  * The pair leaves together (cluster barrier) after the last tile, then frees its tensor memory. All waits bounded. */
 /* A pair's tile is 256 rows x WIDTH features, WIDTH = NSUB * NMMA: NSUB MMAs of N = NMMA per K = 16 step into
  * neighbouring accumulator columns. <256, 1> is the standard tile; <160, 2> (320 wide, one accumulator) exists for

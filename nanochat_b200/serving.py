@@ -142,7 +142,8 @@ class NativeDecoder:
     """Continuous batching over `decoder`'s slots (its n_slots is the batch). A request's tokens depend on neither
     the other requests in the batch nor the slot it lands in: rows of a step never mix (each GEMM row, each attention
     sequence and each choice is computed from that row alone, in an order fixed by the decoder's shape), which the
-    GPU tests check bit for bit. end_token: the token that ends a continuation without being emitted (the
+    GPU tests check bit for bit; a prompt's kernels follow from that prompt alone. (Models of mixed layers choose the
+    kernels of their recurrent layers, and latent or split attention, by the prompts that share a pass: rounding may differ.) end_token: the token that ends a continuation without being emitted (the
     reference's BOS, inference/decoder.py:305-307)."""
 
     def __init__(self, decoder: StepDecoder, *, end_token: int):
