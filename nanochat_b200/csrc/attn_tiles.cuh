@@ -124,6 +124,37 @@ template <bool TRANSPOSED> __device__ __forceinline__ float staged_value(const u
     return __bfloat162float(*reinterpret_cast<const bf16 *>(tile + c / 64 * KEYS * 128 + j * 128 + ((c % 64 / 8 ^ j & 7) * 16) + c % 8 * 2));
 }
 
+/* What the MMAs of a key tile do, by the softmax warps: each thread its row's probabilities (from tensor memory, as the MMA would
+ * read them) times the first `seen` positions' values, added to O. Out of line: the main loop keeps its registers. */
+template <int VB, int P, bool SCALED> __device__ __noinline__ void multiply_rows(const uint8_t *v, uint32_t p_mine, uint32_t o_mine, int seen, bool first) {
+    uint32_t u[KEYS];
+    float p[KEYS];
+    tmem_wait_store();
+    tmem_fetch64(p_mine, u);
+#pragma unroll
+    for (int j = 0; j < KEYS; j += 2) {
+        const uint32_t hi = u[j / 2], lo = u[KEYS / 2 + j / 2];
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+        p[j] = P == P_F16 ? f.x : __uint_as_float(hi << 16) + __uint_as_float(lo << 16);
+        p[j + 1] = P == P_F16 ? f.y : __uint_as_float(hi & 0xffff0000u) + __uint_as_float(lo & 0xffff0000u);
+    }
+#pragma unroll 1
+    for (int c = 0; c < VB * 2; c++) {
+        float o[32] = {};
+        if (!first) tmem_load32(o_mine + c * 32, o);
+#pragma unroll 1
+        for (int j = 0; j < seen; j++)
+#pragma unroll
+            for (int e = 0; e < 32; e++) o[e] = fmaf(p[j], staged_value<SCALED>(v, j, c * 32 + e), o[e]);
+        __syncwarp();
+        uint32_t x[32];
+#pragma unroll
+        for (int e = 0; e < 32; e++) x[e] = __float_as_uint(o[e]);
+        tmem_store16(o_mine + c * 32, x);
+        tmem_store16(o_mine + c * 32 + 16, x + 16);
+    }
+}
+
 /* The block's program. `work()` is called by every thread once the kernel before this one has finished; finish(row, m, l, c, v) gets
  * row `row` of the tile's O (un-normalised, relative to 2^m; l: the sum) 32 columns from c at a time. */
 template <int KB, int VB, int P, bool SCALED, typename GetWork, typename Finish>
@@ -253,7 +284,7 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
         const int last = w.pos0 + min(tid, w.rows - 1); /* the last position the row sees */
         const uint32_t mine = tmem + ((uint32_t)(warp * 32) << 16), o_mine = t_out + ((uint32_t)(warp * 32) << 16);
         float m = 0.f, l = 0.f;
-        bool ok = true;
+        bool ok = true, pending = SCALED; /* some row of the warp may have had no finite score yet */
         for (int i = 0; i < n; i++) {
             ok = wait_all(s_full(i & 1), i >> 1);
             if (!ok) break;
@@ -312,12 +343,14 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                     tmem_store16(o_mine + c * 32 + 16, u + 16);
                 }
             }
-            const bool none = SCALED && m == -INFINITY; /* no finite score so far: nothing counts yet, as in k_prefill_attn */
-            if (SCALED && __any_sync(0xffffffffu, none)) {
+            float reference = m;
+            if (SCALED && pending) {
+                const bool none = m == -INFINITY; /* nothing counts yet, as in k_prefill_attn */
+                pending = __any_sync(0xffffffffu, none);
 #pragma unroll
                 for (int j = 0; j < KEYS; j++) s[j] = none ? -INFINITY : s[j];
+                reference = none ? 0.f : m;
             }
-            const float reference = none ? 0.f : m;
             if (i >= border) {
                 ok = wait_all(v_full(i % S::V_STAGES), i / S::V_STAGES);
                 if (!ok) break;
@@ -366,36 +399,10 @@ __device__ __forceinline__ void attend(uint8_t *raw, int *status, GetWork work, 
                 ok = wait_all(looked, i - border);
                 if (!ok) break;
                 if (odd[i - border]) {
-                    const uint8_t *v = raw + S::AT_V + (i % S::V_STAGES) * S::V_BYTES;
-                    uint32_t u[KEYS];
-                    float p[KEYS]; /* the probabilities as the MMA would have read them */
-                    tmem_wait_store();
-                    tmem_fetch64(p_mine, u);
-#pragma unroll
-                    for (int j = 0; j < KEYS; j += 2) {
-                        const uint32_t hi = u[j / 2], lo = u[KEYS / 2 + j / 2];
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
-                        p[j] = P == P_F16 ? f.x : __uint_as_float(hi << 16) + __uint_as_float(lo << 16);
-                        p[j + 1] = P == P_F16 ? f.y : __uint_as_float(hi & 0xffff0000u) + __uint_as_float(lo & 0xffff0000u);
-                    }
                     ok = i == 0 || wait_all(pv_done((i - 1) & 1), (i - 1) >> 1); /* O is complete up to the tile before */
                     if (!ok) break;
                     fence_after();
-#pragma unroll 1
-                    for (int c = 0; c < VB * 2; c++) {
-                        float o[32] = {};
-                        if (i > 0) tmem_load32(o_mine + c * 32, o);
-#pragma unroll 1
-                        for (int j = 0; j < KEYS && p0 + j <= last; j++)
-#pragma unroll
-                            for (int e = 0; e < 32; e++) o[e] = fmaf(p[j], staged_value<SCALED>(v, j, c * 32 + e), o[e]);
-                        __syncwarp();
-                        uint32_t u[32];
-#pragma unroll
-                        for (int e = 0; e < 32; e++) u[e] = __float_as_uint(o[e]);
-                        tmem_store16(o_mine + c * 32, u);
-                        tmem_store16(o_mine + c * 32 + 16, u + 16);
-                    }
+                    multiply_rows<VB, P, SCALED>(raw + S::AT_V + (i % S::V_STAGES) * S::V_BYTES, p_mine, o_mine, min(last - p0 + 1, KEYS), i == 0);
                 }
             }
             tmem_wait_store();
