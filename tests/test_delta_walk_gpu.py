@@ -14,7 +14,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("sizes", [dict(dim=16, vdim=16, conv=1, heads=1, kv_heads=1), dict(dim=64, vdim=48, heads=4, kv_heads=2), dict(dim=80, vdim=272, heads=2, kv_heads=1),
-                                   dict(dim=128, vdim=128, heads=3, kv_heads=3), dict(dim=144, vdim=32, conv=6, heads=2, kv_heads=2), dict(dim=256, vdim=64, conv=2, heads=2, kv_heads=1)])
+                                   dict(dim=128, vdim=128, heads=3, kv_heads=3), dict(dim=144, vdim=32, conv=6, heads=2, kv_heads=2), dict(dim=256, vdim=64, conv=2, heads=2, kv_heads=1),
+                                   # two and four values per lane at every number of key channels per lane, a last block of values that is not full
+                                   dict(dim=64, vdim=128, heads=4, kv_heads=2), dict(dim=192, vdim=128, heads=4, kv_heads=4), dict(dim=256, vdim=128, heads=4, kv_heads=1),
+                                   dict(dim=64, vdim=128, heads=8, kv_heads=4), dict(dim=128, vdim=144, heads=8, kv_heads=2), dict(dim=192, vdim=128, heads=8, kv_heads=8),
+                                   dict(dim=256, vdim=128, heads=8, kv_heads=2)])
 def test_walk_equals_token_by_token(dtype, sizes):
     entry, C = cases.delta(**sizes), 64
     state = cases.random_state(cases.config([entry], width=C), 61)
