@@ -55,29 +55,57 @@ static __device__ __forceinline__ float group_max(float v) {
     return v;
 }
 
+/* Two fp32 operations as one instruction. Sums of products take their sums one by one: add.rn.f32x2 of mul.rn.f32x2 is contracted
+ * to a fused multiply-add, which rounds once. */
+static __device__ __forceinline__ uint64_t pair_of(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+static __device__ __forceinline__ float2 values_of(uint64_t p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+static __device__ __forceinline__ uint64_t mul2_rn(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+static __device__ __forceinline__ uint64_t fma2_rn(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 /* x1, x2 (this lane's 8 + 8 values) -> normed, gained, rotated values rounded to bf16 and widened again. */
 static __device__ __forceinline__ void norm_rotate(float *x1, float *x2, const float *gain, const float *cs,
                                                    const float *sn, int o) {
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < VEC; i++)
-        ss = __fadd_rn(ss, __fadd_rn(__fmul_rn(x1[i], x1[i]), __fmul_rn(x2[i], x2[i])));
+    for (int i = 0; i < VEC; i += 2) {
+        const uint64_t a = pair_of(x1[i], x1[i + 1]), b = pair_of(x2[i], x2[i + 1]);
+        const float2 s = values_of(mul2_rn(a, a)), u = values_of(mul2_rn(b, b));
+        ss = __fadd_rn(__fadd_rn(ss, __fadd_rn(s.x, u.x)), __fadd_rn(s.y, u.y));
+    }
     ss = group_sum(ss);
     const float mean = __fmul_rn(ss, 1.f / (float)HEAD_DIM); /* a power of two: the same rounding as the division */
     const float r = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(mean, FLT_EPSILON)));
+    const uint64_t rr = pair_of(r, r);
 #pragma unroll
     for (int q = 0; q < VEC; q += 4) { /* four dims and their partners at a time: 16 table values live, not 32 */
         const float4 g1 = *reinterpret_cast<const float4 *>(gain + o + q), g2 = *reinterpret_cast<const float4 *>(gain + HALF + o + q);
-        const float4 c = *reinterpret_cast<const float4 *>(cs + o + q), s = *reinterpret_cast<const float4 *>(sn + o + q);
-        const float g1v[4] = {g1.x, g1.y, g1.z, g1.w}, g2v[4] = {g2.x, g2.y, g2.z, g2.w};
-        const float cv[4] = {c.x, c.y, c.z, c.w}, sv[4] = {s.x, s.y, s.z, s.w};
+        const float4 cc = *reinterpret_cast<const float4 *>(cs + o + q), s = *reinterpret_cast<const float4 *>(sn + o + q);
+        const uint64_t g1v[2] = {pair_of(g1.x, g1.y), pair_of(g1.z, g1.w)}, g2v[2] = {pair_of(g2.x, g2.y), pair_of(g2.z, g2.w)};
+        const uint64_t cv[2] = {pair_of(cc.x, cc.y), pair_of(cc.z, cc.w)}, sv[2] = {pair_of(s.x, s.y), pair_of(s.z, s.w)};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float n1 = __fmul_rn(__fmul_rn(x1[q + i], r), g1v[i]), n2 = __fmul_rn(__fmul_rn(x2[q + i], r), g2v[i]);
-            const float y1 = __fadd_rn(__fmul_rn(n1, cv[i]), __fmul_rn(n2, sv[i]));
-            const float y2 = __fsub_rn(__fmul_rn(n2, cv[i]), __fmul_rn(n1, sv[i]));
-            x1[q + i] = __bfloat162float(__float2bfloat16_rn(y1));
-            x2[q + i] = __bfloat162float(__float2bfloat16_rn(y2));
+        for (int i = 0; i < 2; i++) {
+            const int at = q + 2 * i;
+            const uint64_t n1 = mul2_rn(mul2_rn(pair_of(x1[at], x1[at + 1]), rr), g1v[i]), n2 = mul2_rn(mul2_rn(pair_of(x2[at], x2[at + 1]), rr), g2v[i]);
+            const float2 a = values_of(mul2_rn(n1, cv[i])), b = values_of(mul2_rn(n2, sv[i])), c = values_of(mul2_rn(n2, cv[i])), d = values_of(mul2_rn(n1, sv[i]));
+            const float2 z1 = __bfloat1622float2(__floats2bfloat162_rn(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)));
+            const float2 z2 = __bfloat1622float2(__floats2bfloat162_rn(__fsub_rn(c.x, d.x), __fsub_rn(c.y, d.y)));
+            x1[at] = z1.x, x1[at + 1] = z1.y, x2[at] = z2.x, x2[at + 1] = z2.y;
         }
     }
 }
@@ -157,11 +185,12 @@ static __device__ __forceinline__ float quantise(const float *x1, const float *x
     float q1[VEC], q2[VEC];
     if (amax > 0x1p-100f && amax < 0x1p100f) {
         const float r = __frcp_rn(scale);
+        const uint64_t rr = pair_of(r, r), minus = pair_of(-scale, -scale);
 #pragma unroll
-        for (int i = 0; i < VEC; i++) {
-            const float a1 = __fmul_rn(x1[i], r), a2 = __fmul_rn(x2[i], r);
-            q1[i] = __fmaf_rn(__fmaf_rn(-scale, a1, x1[i]), r, a1);
-            q2[i] = __fmaf_rn(__fmaf_rn(-scale, a2, x2[i]), r, a2);
+        for (int i = 0; i < VEC; i += 2) {
+            const uint64_t u1 = pair_of(x1[i], x1[i + 1]), u2 = pair_of(x2[i], x2[i + 1]), a1 = mul2_rn(u1, rr), a2 = mul2_rn(u2, rr);
+            const float2 f1 = values_of(fma2_rn(fma2_rn(minus, a1, u1), rr, a1)), f2 = values_of(fma2_rn(fma2_rn(minus, a2, u2), rr, a2));
+            q1[i] = f1.x, q1[i + 1] = f1.y, q2[i] = f2.x, q2[i + 1] = f2.y;
         }
     } else {
 #pragma unroll

@@ -173,3 +173,17 @@ def test_prefill_runs_store_the_same_bytes_as_single_rows():
         for p in range(192):
             if (slot, p) not in written:
                 assert not k[:, p].any() and not v[:, p].any() and not ks[:, p].any() and not vs[:, p].any(), (slot, p)
+
+
+@pytest.mark.parametrize("hidden", [0, 256])
+@pytest.mark.parametrize("starts", [list(range(16)), [15, 0, 7, 3], [16, 1]])
+@pytest.mark.parametrize("length", [1, 15, 16, 17, 31, 47])
+def test_groups_of_sixteen_anywhere_in_a_pass(length, starts, hidden):
+    """Prompts one behind the other whose first rows fall anywhere in a block and on any position: the 16 positions that share a
+    chunk lie in one block, across two, or are not all there; descending positions and a slot change inside a group as well."""
+    slots = [s for s, a in enumerate(starts) for _ in range(length)]
+    positions = [a + i for a in starts for i in range(length)]
+    n = len(starts)
+    slots += [n] * 32 + [n + i // 16 for i in range(32)]  # backwards; 16 positions of two slots after a jump
+    positions += list(range(95, 63, -1)) + [8 + i % 16 for i in range(32)]
+    run_case(seed=900 + length, rows=len(slots), Hq=4, Hkv=2, max_len=128, n_slots=n + 2, positions=positions, slots=slots, ve_hidden=hidden)
