@@ -12,7 +12,7 @@
  *     shared-memory stages with cp.async.bulk.tensor (TMA, 128-byte swizzle, no multicast); weight loads for the
  *     first ring fill are issued BEFORE griddepcontrol.wait, so in a captured step the stream starts under the
  *     predecessor's tail;
- *   - thread 32 issues tcgen05.mma.cta_group::1.kind::f16 (4 per k-block) and releases stages with tcgen05.commit;
+ *   - warp 1, one lane of it, issues tcgen05.mma.cta_group::1.kind::f16 (4 per k-block) and releases stages with tcgen05.commit;
  *   - warps 2, 3 sum the squares of the staged x boxes for the fused norm. The norm has no gain, so
  *     norm(x) . W^T = rstd[row] * (x . W^T): the scale is applied to the fp32 accumulators in the epilogue.
  * K is split over a thread-block cluster of up to 8 blocks so that short-and-wide projections (16 feature tiles of
@@ -173,27 +173,31 @@ __global__ void __launch_bounds__(THREADS) k_stream_gemm(const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) { /* MMA issuer */
-            constexpr uint32_t IDESC = (1u << 4) /* fp32 accumulators */ | (1u << 7) /* A bf16 */ | (1u << 10) /* B bf16 */
-                                       | ((uint32_t)(NP >> 3) << 17) | ((uint32_t)(TILE_F >> 4) << 24); /* both K-major */
-            bool ok = true;
-            for (int i = 0; i < nst; i++) {
-                const int s = i % STAGES, n = boxes_of(i);
-                ok = mbar_wait(full(s), (i / STAGES) & 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = ring + s * Sh::STAGE_BYTES, b_addr = a_addr + KSUB * A_BOX_BYTES;
+        /* MMA issuer: the warp goes through the loop together (elect_one) */
+        constexpr uint32_t IDESC = (1u << 4) /* fp32 accumulators */ | (1u << 7) /* A bf16 */ | (1u << 10) /* B bf16 */
+                                   | ((uint32_t)(NP >> 3) << 17) | ((uint32_t)(TILE_F >> 4) << 24); /* both K-major */
+        const uint32_t acc = __shfl_sync(0xffffffffu, tmem, 0), stages = __shfl_sync(0xffffffffu, ring, 0);
+        bool ok = true;
+        for (int i = 0; i < nst; i++) {
+            const int s = i % STAGES, n = boxes_of(i);
+            ok = __all_sync(0xffffffffu, mbar_wait(full(s), (i / STAGES) & 1));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = stages + s * Sh::STAGE_BYTES, b_addr = a_addr + KSUB * A_BOX_BYTES;
+            if (elect_one()) {
                 for (int b = 0; b < n; b++) {
 #pragma unroll
                     for (int k = 0; k < KBLK / 16; k++) /* 16 k-values = 32 bytes further along the swizzled row */
-                        umma_bf16(tmem, umma_desc(a_addr + b * A_BOX_BYTES + k * 32),
+                        umma_bf16(acc, umma_desc(a_addr + b * A_BOX_BYTES + k * 32),
                                   umma_desc(b_addr + b * Sh::B_BOX_BYTES + k * 32), IDESC, (i | b | k) != 0);
                 }
                 umma_commit(empty(s));
             }
-            if (!ok) flag(a.status, NCB_DEV_WAIT_TIMEOUT);
-            umma_commit(accum_bar);
+            __syncwarp();
         }
+        if (!ok && lane == 0) flag(a.status, NCB_DEV_WAIT_TIMEOUT);
+        if (elect_one()) umma_commit(accum_bar);
+        __syncwarp();
     }
     if (tid != 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp >= 2 && !a.norm_input) { /* row scales from the stream's partial sums; every block needs every row's */

@@ -10,7 +10,7 @@
  * accumulators in tensor memory. One persistent block per SM walks over the output tiles:
  *   - warp 0, one thread: TMA producer. Per 64-wide k-block one box of x (128 rows) and one of W (BN rows) into a ring
  *     of shared-memory stages (cp.async.bulk.tensor, 128-byte swizzle, no multicast), one mbarrier per stage;
- *   - warp 1, one thread: issues tcgen05.mma.cta_group::1.kind::f16 (four K = 16 steps per k-block), releases stages
+ *   - warp 1, one lane: issues tcgen05.mma.cta_group::1.kind::f16 (four K = 16 steps per k-block), releases stages
  *     with tcgen05.commit, and signals a finished accumulator. Tensor memory holds TWO accumulators (2 x BN columns), so
  *     the MMAs of the next tile run while the epilogue drains the previous one;
  *   - warps 2..5: epilogue. Warp w owns the 32 tensor-memory lanes (= rows) its rank allows (w % 4), a thread reads
@@ -299,38 +299,43 @@ __global__ void __launch_bounds__(threads_of(EPI), 1) k_tile_gemm(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) { /* MMA issuer */
+        { /* MMA issuer: the warp goes through the loop together (elect_one) */
             constexpr uint32_t IDESC_BASE = (1u << 4) /* fp32 accumulators */ | (1u << 7) /* A bf16 */ | (1u << 10) /* B bf16 */
                                             | ((uint32_t)(BM >> 4) << 24); /* both K-major; N goes to bits 17.. */
+            const uint32_t accs = __shfl_sync(0xffffffffu, tmem, 0), stages = __shfl_sync(0xffffffffu, ring, 0);
             uint32_t g = 0, it = 0;
-            for (int u = blockIdx.x; u < units && !*failed; u += gridDim.x, it++) {
+            for (int u = blockIdx.x; u < units && !__any_sync(0xffffffffu, *failed); u += gridDim.x, it++) {
                 const uint32_t buf = it & 1;
                 const uint32_t idesc = IDESC_BASE | ((uint32_t)(unit_of<BN>(u, n_tiles, split_from).width >> 3) << 17);
-                if (!mbar_wait(acc_empty(buf), ((it >> 1) & 1) ^ 1)) { /* the epilogue has drained this accumulator */
+                if (!__all_sync(0xffffffffu, mbar_wait(acc_empty(buf), ((it >> 1) & 1) ^ 1))) { /* the epilogue has drained this accumulator */
                     flag(a.status, NCB_DEV_WAIT_TIMEOUT);
                     *failed = 1;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + buf * BN;
+                const uint32_t acc = accs + buf * BN;
                 bool ok = true;
                 for (int kb = 0; kb < nkb; kb++, g++) {
                     const int s = g % STAGES;
-                    ok = mbar_wait(full(s), (g / STAGES) & 1);
+                    ok = __all_sync(0xffffffffu, mbar_wait(full(s), (g / STAGES) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = ring + s * T::STAGE_BYTES, b_addr = a_addr + A_BYTES;
+                    const uint32_t a_addr = stages + s * T::STAGE_BYTES, b_addr = a_addr + A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < KBLK / 16; k++) /* 16 k-values = 32 bytes further along the swizzled row */
-                        umma_bf16(acc, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc, (kb | k) != 0);
-                    umma_commit(empty(s));
+                        for (int k = 0; k < KBLK / 16; k++) /* 16 k-values = 32 bytes further along the swizzled row */
+                            umma_bf16(acc, umma_desc(a_addr + k * 32), umma_desc(b_addr + k * 32), idesc, (kb | k) != 0);
+                        umma_commit(empty(s));
+                    }
+                    __syncwarp();
                 }
                 if (!ok) {
                     flag(a.status, NCB_DEV_WAIT_TIMEOUT);
                     *failed = 1;
                     break;
                 }
-                umma_commit(acc_full(buf));
+                if (elect_one()) umma_commit(acc_full(buf));
+                __syncwarp();
             }
         }
     } else { /* epilogue warps 2..5 (2..9): tensor-memory lanes 32 (warp % 4) .. + 31 */
@@ -547,43 +552,48 @@ __global__ void __launch_bounds__(threads_of(EPI), 1) k_tile_gemm_pair(const __g
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) { /* MMA issuer of the pair */
+        if (rank == 0) { /* MMA issuer of the pair: the warp goes through the loop together (elect_one) */
             constexpr uint32_t IDESC_BASE = (1u << 4) /* fp32 accumulators */ | (1u << 7) /* A bf16 */ | (1u << 10) /* B bf16 */
                                             | ((uint32_t)((2 * BM) >> 4) << 24); /* M 256 over the pair */
+            const uint32_t accs = __shfl_sync(0xffffffffu, tmem, 0), stages = __shfl_sync(0xffffffffu, ring, 0);
             uint32_t g = 0, it = 0;
-            for (int u = pair; u < units && !*failed; u += n_pairs, it++) {
+            for (int u = pair; u < units && !__any_sync(0xffffffffu, *failed); u += n_pairs, it++) {
                 const uint32_t buf = acc_of(it);
                 const bool whole = pair_unit_of<WIDTH>(u, n_tiles, split_from).width == WIDTH;
                 const uint32_t idesc = IDESC_BASE | ((uint32_t)((whole ? NMMA : NMMA / 2) >> 3) << 17);
-                if (!mbar_wait(acc_empty(buf), (use_of(it) & 1) ^ 1)) { /* both blocks have drained this accumulator */
+                if (!__all_sync(0xffffffffu, mbar_wait(acc_empty(buf), (use_of(it) & 1) ^ 1))) { /* both blocks have drained this accumulator */
                     flag(a.status, NCB_DEV_WAIT_TIMEOUT);
                     *failed = 1;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc = tmem + buf * WIDTH;
+                const uint32_t acc = accs + buf * WIDTH;
                 bool ok = true;
                 for (int kb = 0; kb < nkb; kb++, g++) {
                     const int s = g % STAGES;
-                    ok = mbar_wait(full(s), (g / STAGES) & 1);
+                    ok = __all_sync(0xffffffffu, mbar_wait(full(s), (g / STAGES) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = ring + s * P::STAGE_BYTES, b_addr = a_addr + A_BYTES;
+                    const uint32_t a_addr = stages + s * P::STAGE_BYTES, b_addr = a_addr + A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < KBLK / 16; k++)
+                        for (int k = 0; k < KBLK / 16; k++)
 #pragma unroll
-                        for (int j = 0; j < NSUB; j++)
-                            if (j == 0 || whole)
-                                umma_bf16_pair(acc + j * NMMA, umma_desc(a_addr + k * 32),
-                                               umma_desc(b_addr + j * P::SUB_BYTES + k * 32), idesc, (kb | k) != 0);
-                    umma_commit_pair(empty(s));
+                            for (int j = 0; j < NSUB; j++)
+                                if (j == 0 || whole)
+                                    umma_bf16_pair(acc + j * NMMA, umma_desc(a_addr + k * 32),
+                                                   umma_desc(b_addr + j * P::SUB_BYTES + k * 32), idesc, (kb | k) != 0);
+                        umma_commit_pair(empty(s));
+                    }
+                    __syncwarp();
                 }
                 if (!ok) {
                     flag(a.status, NCB_DEV_WAIT_TIMEOUT);
                     *failed = 1;
                     break;
                 }
-                umma_commit_pair(acc_full(buf));
+                if (elect_one()) umma_commit_pair(acc_full(buf));
+                __syncwarp();
             }
         }
     } else { /* epilogue warps 2..5 (2..9) of both blocks: this block's tensor-memory lanes 32 (warp % 4) .. + 31 */

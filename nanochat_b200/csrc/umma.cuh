@@ -43,6 +43,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (clock64() - start > WAIT_CYCLES) return false;
     }
 }
+/* True for one lane (always the same) of a warp that is together here: the lane that issues MMAs and their commits. With `lane == 0` in
+ * its place the compiler does not keep what an MMA takes in uniform registers, and issuing one takes 66 to 69 cycles whatever its
+ * size; so 43 (N = 32), 49 (64) or 64 (128: the tensor cores' own rate). The 320-wide tiles of tile_gemm (two MMAs of N = 160 a pair),
+ * 4,088 rows, 1,280 wide, K 3,072: 38.0 -> 34.3 us with an fp32 stream, 51.1 -> 46.6 with two; stream_gemm 0.2 to 0.5 us a launch. */
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "elect.sync _|p, 0xffffffff;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(p));
+    return p;
+}
 /* One box of a 2-d tensor map into shared memory; (c0, c1) = (k, row) element coordinates, c0 a multiple of 64.
  * `policy` is an L2 eviction policy: weights are read once (evict first), activations by every block (evict last). */
 __device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar, uint64_t policy) {
