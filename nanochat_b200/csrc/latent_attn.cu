@@ -23,6 +23,7 @@
  */
 #include "attn_tiles.cuh"
 
+#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -496,21 +497,25 @@ template <typename T> __global__ void __launch_bounds__(THREADS) k_latent_out_an
     }
 }
 
-constexpr int OUT_THREADS = 256;
+constexpr int OUT_THREADS = 256, OUT_ROWS = 4;
 
-/* Grid (slices, heads, ceil(rows / 16)), cluster (slices, 1, 1): a block merges rank / slices latent columns of 16 rows,
+/* Grid (slices, heads, ceil(rows / 4)), cluster (slices, 1, 1): a block merges rank / slices latent columns of 4 rows,
  * multiplies them by its columns of W_uv (on their way to shared memory before the dependency wait) for all of the head's
- * values, and the cluster adds the partial products up. */
+ * values, and the cluster adds the partial products up. Bound by the chain of loads of the longest rows' states, so few rows share a
+ * block and its weights (which come from L2) although the product's M is 16: 32 rows of 256 to 8,192 positions, longest first, 16
+ * heads: 19.0 -> 13.5 us a launch (16 rows per block before). */
 __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) {
     extern __shared__ __align__(128) uint8_t raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int slices = gridDim.x, rank_block = blockIdx.x, h = blockIdx.y, r0 = blockIdx.z * 16;
+    const int slices = gridDim.x, rank_block = blockIdx.x, h = blockIdx.y, r0 = blockIdx.z * OUT_ROWS;
     const int cols = a.rank / slices, c0 = rank_block * cols, xs = cols + 8, V = a.vdim;
-    float *w = reinterpret_cast<float *>(raw);                          /* [16][max_chunks] */
-    float *sum = w + 16 * a.max_chunks;                                 /* [16][vdim + 4] partial products */
-    bf16 *x = reinterpret_cast<bf16 *>(sum + 16 * (V + 4));             /* [16][cols + 8] merged latent */
-    bf16 *u = x + 16 * xs;                                              /* [vdim][cols + 8] */
-    __shared__ int n_chunks[16];
+    const int items = OUT_ROWS * (cols / 4), shares = max(1, min(OUT_THREADS / items, 4)); /* threads that share an item's states */
+    float *w = reinterpret_cast<float *>(raw);                                          /* [4][max_chunks, a multiple of 4] */
+    float *sum = w + OUT_ROWS * ((a.max_chunks + 3) & ~3);                              /* [4][vdim + 4] partial products */
+    float4 *part = reinterpret_cast<float4 *>(sum + OUT_ROWS * (V + 4));                /* [shares - 1][items] */
+    bf16 *x = reinterpret_cast<bf16 *>(part + (shares - 1) * items);                    /* [4][cols + 8] merged latent */
+    bf16 *u = x + OUT_ROWS * xs;                                                        /* [vdim][cols + 8] */
+    __shared__ int n_chunks[OUT_ROWS];
     {
         const int per = cols / 8;
         const bf16 *src = (const bf16 *)a.w_uv + (size_t)h * V * a.rank + c0;
@@ -519,38 +524,39 @@ __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) 
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int rows = (int)(a.rows - r0 < 16 ? a.rows - r0 : 16);
+    const int rows = (int)(a.rows - r0 < OUT_ROWS ? a.rows - r0 : OUT_ROWS);
     const size_t state = (size_t)(a.rank + STATE_PAD);
-    { /* the factor of every chunk's state, 16 threads per row: 2^(m - M) / L with the sink in M and L */
-        const int r = tid >> 4, j = tid & 15;
+    const int ws = (a.max_chunks + 3) & ~3;
+    if (warp < OUT_ROWS) { /* the factor of every chunk's state, a warp per row: 2^(m - M) / L with the sink in M and L */
+        const int r = warp;
         int n = 0, slot;
         if (r < rows) n = cut_of(length_of(a, r0 + r, slot), a.chunk_tiles).n_chunks;
         const float *p = a.parts + ((size_t)(r0 + r) * a.heads + h) * a.max_chunks * state;
         const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
         float M = sink, L = 0.f;
-        for (int c = j; c < n; c += 16) M = fmaxf(M, p[c * state]);
-        for (int o = 8; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        for (int c = j; c < n; c += 16) {
+        for (int c = lane; c < n; c += 32) M = fmaxf(M, p[c * state]);
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        for (int c = lane; c < n; c += 32) {
             const float2 ml = *reinterpret_cast<const float2 *>(p + c * state);
             const float e = exp2f(ml.x - M);
-            w[r * a.max_chunks + c] = e;
+            w[r * ws + c] = e;
             L = fmaf(e, ml.y, L);
         }
-        for (int o = 8; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
         if (a.sink) L += exp2f(sink - M);
         const float inv = n > 0 ? 1.f / L : 0.f;
-        for (int c = j; c < n; c += 16) w[r * a.max_chunks + c] *= inv;
-        if (j == 0) n_chunks[r] = n;
+        for (int c = lane; c < n; c += 32) w[r * ws + c] *= inv;
+        if (lane == 0) n_chunks[r] = n;
     }
     __syncthreads();
-    for (int i = tid; i < 16 * (cols / 4); i += OUT_THREADS) {
-        const int r = i / (cols / 4), c4 = i % (cols / 4) * 4;
+    for (int at = tid; at < items * shares; at += OUT_THREADS) { /* (shares > 1: every thread has one item at most) */
+        const int i = at % items, share = at / items, r = i / (cols / 4), c4 = i % (cols / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         const int n = n_chunks[r];
         const float *p = a.parts + ((size_t)(r0 + r) * a.heads + h) * a.max_chunks * state + STATE_PAD + c0 + c4;
-        const float *f = w + r * a.max_chunks;
+        const float *f = w + r * ws;
         constexpr int AHEAD = 8; /* states whose loads are in flight together */
-        for (int c = 0; c < n; c += AHEAD) {
+        for (int c = share * AHEAD; c < n; c += shares * AHEAD) {
             float4 s[AHEAD];
 #pragma unroll
             for (int j = 0; j < AHEAD; j++)
@@ -561,23 +567,30 @@ __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) 
                 v.x = fmaf(e, s[j].x, v.x), v.y = fmaf(e, s[j].y, v.y), v.z = fmaf(e, s[j].z, v.z), v.w = fmaf(e, s[j].w, v.w);
             }
         }
+        if (share) part[(share - 1) * items + i] = v;
+        if (shares > 1) {
+            asm volatile("bar.sync 1, %0;" ::"r"(items * shares) : "memory"); /* whole warps: items are a multiple of 32 */
+            if (share) continue;
+            for (int k = 0; k < shares - 1; k++) {
+                const float4 o = part[k * items + i];
+                v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
+            }
+        }
         *reinterpret_cast<uint2 *>(x + r * xs + c4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int n0 = warp * 8; n0 < V; n0 += OUT_THREADS / 4) { /* 8 output values at a time */
+    for (int n0 = warp * 8; n0 < V; n0 += OUT_THREADS / 4) { /* 8 output values at a time; rows past the fourth are zeros */
         float acc[2][4] = {};
-        const bf16 *wr = u + (n0 + g) * xs + 8 * t, *xl = x + g * xs + 8 * t, *xh = xl + 8 * xs;
+        const bf16 *wr = u + (n0 + g) * xs + 8 * t, *xl = x + g * xs + 8 * t;
 #pragma unroll 4
         for (int k = 0; k < cols; k += 32) {
-            const uint4 lo = *reinterpret_cast<const uint4 *>(xl + k), hi = *reinterpret_cast<const uint4 *>(xh + k);
+            const uint4 lo = g < OUT_ROWS ? *reinterpret_cast<const uint4 *>(xl + k) : make_uint4(0u, 0u, 0u, 0u);
             const uint4 b = *reinterpret_cast<const uint4 *>(wr + k);
-            mma_bf16(acc[0], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
-            mma_bf16(acc[1], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
+            mma_bf16(acc[0], lo.x, 0u, lo.y, 0u, b.x, b.y);
+            mma_bf16(acc[1], lo.z, 0u, lo.w, 0u, b.z, b.w);
         }
-        float *s = sum + n0 + 2 * t;
-        *reinterpret_cast<float2 *>(s + g * (V + 4)) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
-        *reinterpret_cast<float2 *>(s + (g + 8) * (V + 4)) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+        if (g < OUT_ROWS) *reinterpret_cast<float2 *>(sum + g * (V + 4) + n0 + 2 * t) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
     }
     cg::cluster_group cluster = cg::this_cluster();
     if (slices > 1) cluster.sync();
@@ -929,9 +942,11 @@ int latent_out(const ncb_latent *g, int f32, void *stream) {
     if (!f32) {
         int slices = 4;
         while (slices > 1 && g->rank % (slices * 32)) slices /= 2;
-        const size_t smem = (size_t)16 * g->max_chunks * 4 + (size_t)16 * (g->vdim + 4) * 4 + (size_t)(16 + g->vdim) * (g->rank / slices + 8) * 2;
+        const int cols = g->rank / slices, items = OUT_ROWS * (cols / 4), shares = std::max(1, std::min(OUT_THREADS / items, 4));
+        const size_t smem = (size_t)OUT_ROWS * ((g->max_chunks + 3) / 4 * 4) * 4 + (size_t)OUT_ROWS * (g->vdim + 4) * 4 + (size_t)(shares - 1) * items * 16 +
+                            (size_t)(OUT_ROWS + g->vdim) * (cols + 8) * 2;
         if (smem <= 200 * 1024)
-            return launch(k_latent_out, dim3(slices, g->heads, (unsigned)((g->rows + 15) / 16)), smem, OUT_THREADS, slices, s, *g);
+            return launch(k_latent_out, dim3(slices, g->heads, (unsigned)((g->rows + OUT_ROWS - 1) / OUT_ROWS)), smem, OUT_THREADS, slices, s, *g);
     }
     const size_t smem = ((size_t)g->max_chunks + g->rank) * sizeof(float);
     if (smem > 200 * 1024) return NCB_ERR_UNSUPPORTED;
