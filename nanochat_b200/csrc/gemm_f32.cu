@@ -4,15 +4,16 @@
  * epilogues as the bf16 GEMM libraries (ncb_gemm_rs).
  *
  * Bound by the FMA rate for tens of rows and more, by the weights' way from HBM for a few. A block has a tile of TM rows x 64
- * features and 256 threads, which hold 8 x 8 products each: TM threads cover the tile, so 256 / TM groups of threads share the
+ * features and 128 threads (two blocks per SM), which hold 8 x 8 products each: TM threads cover the tile, so 128 / TM groups share the
  * tile's depth, and every k-value that is loaded from shared memory is used eight times. Both operands arrive as they lie in
  * memory (rows of 64 k-values, 4 floats of padding: rows 4 banks apart) by cp.async into a ring; a thread's four k-values of a
  * row are one 16-byte load and two fma.rn.f32x2 (even and odd k in halves of one register pair, added at the end). What is left
  * is to fill the SMs: narrow products split their depth over a cluster of up to 8 blocks, whose sums meet in a fixed order
  * through distributed shared memory, as in stream_gemm.cu.
- * Measured, us, against 64 x 64 tiles of 4 x 4 products per thread with one buffer and no split: 300 rows, N 3840 K 768 110 -> 76, N 768
- * K 1920 93 -> 33, N 768 K 768 39 -> 16; one row, N 768 K 1920 84 -> 6.7, N 65536 K 768 188 -> 72 (2.8 TB/s); 1024 rows, N 4096 K 1024
- * 254 -> 223 (38.5 TFLOP/s: a thread's 16 loads of 16 bytes per 128 paired multiply-adds keep shared memory as busy as the FMA pipe).
+ * Measured, us, against 64 x 64 tiles of 4 x 4 products per thread with one buffer and no split: 300 rows, N 3840 K 768 110 -> 62, N 768
+ * K 1920 93 -> 35, N 768 K 768 39 -> 17; one row, N 768 K 1920 84 -> 6.3, N 65536 K 768 188 -> 52 (3.9 TB/s); 1024 rows, N 4096 K 1024
+ * 254 -> 213 (40 TFLOP/s: a thread's 16 loads of 16 bytes per 128 paired multiply-adds keep shared memory as busy as the FMA pipe).
+ * One block of 256 threads per SM: 76, 33, 16, 6.7, 72, 223.
  */
 #include "gemm_rs.cuh"
 
@@ -24,7 +25,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int TN = 64, TK = 64, THREADS = 256;
+constexpr int TN = 64, TK = 64, THREADS = 128;
 constexpr int LD = TK + 4;      /* floats from one staged row to the next */
 constexpr int RED_LD = TN + 8;  /* and from one row of products to the next while groups are summed */
 enum { EPI_STORE = 0, EPI_F32 = 3, EPI_GEGLU = 5, EPI_STREAM = 6, EPI_STREAMS = 7, EPI_SWIGLU = 8 };
@@ -86,7 +87,7 @@ __device__ __forceinline__ void finish(const Args &a, long long row, int n, bool
 }
 
 /* Grid (S x row tiles, N / 64), cluster (S, 1, 1): block (m S + s, n) multiplies chunks [s nk / S, (s + 1) nk / S) of the depth. */
-template <int TM> __global__ void __launch_bounds__(THREADS, 1) k_gemm_f32(const Args a, int S) {
+template <int TM> __global__ void __launch_bounds__(THREADS, 2) k_gemm_f32(const Args a, int S) {
     using Sh = Shape<TM>;
     extern __shared__ __align__(128) float ring[];
     __shared__ float factor[TM];
@@ -142,7 +143,7 @@ template <int TM> __global__ void __launch_bounds__(THREADS, 1) k_gemm_f32(const
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float *xs = ring + c % Sh::STAGES * Sh::STAGE + ty * LD + group * Sh::PER;
         const float *ws = ring + c % Sh::STAGES * Sh::STAGE + (TM + tx) * LD + group * Sh::PER;
-#pragma unroll 1
+#pragma unroll
         for (int k = 0; k < Sh::PER; k += 4) {
             float4 wv[8];
 #pragma unroll
