@@ -475,3 +475,21 @@ def test_prefill_attention_groups_rows_and_matches_the_row_wise_path(Hq, Hkv):
                                    [case["k_scale"][b][:, :n]], [case["v_bytes"][b][:, :n]], [case["v_scale"][b][:, :n]], SCALE)
         max_abs, mean_abs = helpers.error_stats(helpers.bf16_bits(got[r:r + 1].cpu()), ref)
         assert max_abs <= 2e-2 and mean_abs <= 2e-3, (r, max_abs, mean_abs)
+
+
+@pytest.mark.parametrize("window", [0, 200])
+@pytest.mark.parametrize("chunk_pages", [2, 3, 5])
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 2), (16, 2)])
+def test_chunks_that_join_in_a_cluster_give_the_merge_launch_s_bits(heads, kv_heads, chunk_pages, window):
+    """Grids that fit the GPU at once with at most eight chunks merge their states in clusters; the same states through the merge launch
+    give the same bits. Rows of no, one and all chunks (with a stub at the end), an empty and an idle one."""
+    lens = [900, 1, 64 * chunk_pages, 64 * chunk_pages + 1, 0, 577]
+    case = helpers.attention_case(950 + heads, heads, kv_heads, lens)
+    cache, q = load_cache(case, max(lens)), helpers.bits_bf16(case["q"]).cuda()
+    lens_t = torch.tensor(lens[:-1] + [-1], dtype=torch.int32, device="cuda")
+    args = dict(max_kv_len=max(lens), window=window, chunk_pages=chunk_pages)
+    out = torch.full(q.shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    ncb.decode_attention(q, cache, lens_t, out=out, **args)
+    part = ncb.decode_attention_partial(q, cache, lens_t, **args)
+    want = ncb.merge_partials(part[None].contiguous())
+    assert torch.equal(out, want) and not out[4:].any() and bool(out[:4].any())
