@@ -806,7 +806,12 @@ static int run_tile_gemm(const void *x, const void *w, TileArgs a, int epilogue,
     const int rows = a.rows, N = a.N, K = a.K;
     CUtensorMap map_x, map_w, map_w_half;
     const bool wide_ok = N % 320 == 0, std_ok = N % 256 == 0;
-    if ((form == 2 || (form == 0 && PAIR_BY_DEFAULT && rows > BM)) && (wide_ok || std_ok)) {
+    /* 128 x 128 tiles, one block each, while one round of the SMs takes them all: a block's operands come at about 55 bytes a cycle
+     * whatever the tile, so few large tiles leave the rest of the chip's loads unused. 1,280 wide, us, pairs -> these: K 1,280, 300 rows
+     * 11.8 -> 9.2, 1,500 12.3 -> 10.1; K 5,120, 300 29.0 -> 25.2, 1,000 30.0 -> 27.4; 3,840 wide, K 1,280, 500 13.3 -> 10.7. In a second
+     * round they lose: 1,280 wide, K 5,120, 2,048 rows (160 tiles) 33.6 -> 47.6; 3,840, 700 rows (180) 14.2 -> 16.0. */
+    const bool small = form == 0 && (long long)((rows + BM - 1) / BM) * (N / 128) <= sm_count_now();
+    if (!small && (form == 2 || (form == 0 && PAIR_BY_DEFAULT && rows > BM)) && (wide_ok || std_ok)) {
         const int pairs = resident_pairs();
         if (pairs > 0) {
             const bool wide = wide_ok && (!std_ok || pair_cost(rows, N, 320, false, pairs) < pair_cost(rows, N, 256, true, pairs));
@@ -821,7 +826,7 @@ static int run_tile_gemm(const void *x, const void *w, TileArgs a, int epilogue,
     } else if (form == 2) {
         return NCB_ERR_UNSUPPORTED;
     }
-    const int bn = N % 256 == 0 ? 256 : 128;
+    const int bn = N % 256 == 0 && !small ? 256 : 128;
     if (!tensor_map(x, rows, K, BM, &map_x) || !tensor_map(w, N, K, bn, &map_w) || !tensor_map(w, N, K, bn / 2, &map_w_half))
         return NCB_ERR_LAUNCH;
     return bn == 256 ? launch_epi<256>(map_x, map_w, map_w_half, a, epilogue, stream)
@@ -838,7 +843,8 @@ extern "C" {
  *   NCB_DEV_WAIT_TIMEOUT is or-ed in if a bounded wait expired. Launched with programmatic stream serialisation.
  *   form: 1 one block per 128 x 256 (or 128 x 128) tile; 2 a pair of blocks per 256 x 256 or 256 x 320 tile (N a
  *   multiple of 256 or of 640, else NCB_ERR_UNSUPPORTED; the width with fewer, fuller rounds of tiles is taken);
- *   0 the pair form where it applies and there are more than 128 rows, else form 1.
+ *   0 one block per 128 x 128 tile where one round of the SMs takes all of them, else the pair form where it applies and there
+ *   are more than 128 rows, else form 1.
  *   All forms give the same bits: a product's k-blocks are accumulated in the same order.
  */
 int tile_gemm_form(const void *x, const void *w, const void *resid, void *y, long long rows, int N, int K, int epilogue,

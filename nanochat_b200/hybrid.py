@@ -17,7 +17,7 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor
 
-from .decoder import StepDecoder
+from .decoder import StepDecoder, streamed
 from .kv_cache import cache_pages
 from .mixers import MIXERS, RowPlan, Rows, pad_to, up
 from .native import MAX_STREAMS, GemmRs, check, cuda_library, pointer, stream
@@ -271,13 +271,13 @@ class HybridDecoder(StepDecoder):
     # ---- GEMMs on the stream ------------------------------------------------------------------------------------------
 
     def gemm_kernel(self, rows: int, N: int, K: int) -> str:
-        """As in decoder.py: up to 16 rows skinny_gemm where it is instantiated for the depth, up to 64 stream_gemm, else
-        tile_gemm; gemm_f32 for a 32-bit model."""
+        """As in decoder.py: up to 16 rows skinny_gemm where it is instantiated for the depth, up to 64 (and beyond where `streamed` says so)
+        stream_gemm, else tile_gemm; gemm_f32 for a 32-bit model."""
         if self.f32:
             return "f32"
         if rows <= 16 and cuda_library("decode_step").skinny_gemm_supported(rows, N, K, 0):
             return "skinny"
-        return "stream" if rows <= 64 else "tile"
+        return "stream" if rows <= 64 or streamed(rows, N, K) else "tile"
 
     ENTRY = {"f32": ("gemm_f32", "gemm_f32_rs", 64), "skinny": ("decode_step", "skinny_gemm_rs", 8),
              "stream": ("stream_gemm", "stream_gemm_rs", 128), "tile": ("tile_gemm", "tile_gemm_rs", 32)}
