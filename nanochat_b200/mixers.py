@@ -74,6 +74,13 @@ class RowPlan:
         self.first, self.count = first, np.diff(np.append(first, n)).astype(np.int32)
         self.slots, self.starts, self.device = slots[first], positions[first], device
         self._on_device: dict = {}
+        self._found: dict = {}
+
+    def once(self, key, make):
+        """make(), kept under `key` for the pass's other layers."""
+        if key not in self._found:
+            self._found[key] = make()
+        return self._found[key]
 
     @property
     def n_segments(self) -> int:
@@ -81,7 +88,7 @@ class RowPlan:
 
     @property
     def longest(self) -> int:
-        return int(self.count.max())
+        return self.once("longest", lambda: int(self.count.max()))
 
     def upload(self, key, arrays: list[np.ndarray]) -> list[Tensor]:
         """The arrays on the device (one copy), kept under `key` for the pass's other layers."""
@@ -96,12 +103,22 @@ class RowPlan:
     def contexts(self) -> list[Tensor]:
         """[segment's slot, first row of its context (n + 1)]: the contexts (all positions up to the segment's end) laid
         out one after the other."""
-        return self.upload("contexts", [self.slots, np.concatenate([[0], np.cumsum(self.starts + self.count)])])
+        return self.once("contexts", lambda: self.upload("contexts", [self.slots, np.concatenate([[0], np.cumsum(self.starts + self.count)])]))
+
+    def extent(self) -> tuple[int, int, float]:
+        """(positions of all contexts together, of the longest, pairs of a row and a position it sees)."""
+        def make():
+            count, length = self.count.astype(np.float64), (self.starts + self.count).astype(np.float64)
+            return int(length.sum()), int(length.max()), float((count * (length - count / 2)).sum())
+        return self.once("extent", make)
 
     def row_tiles(self, size: int, at_least: int = 1, below: int = 1 << 31) -> tuple[list[Tensor], int]:
         """([tile's first row, its rows, its context's first row, its first position], number of tiles) of at most `size`
         rows of one segment, those that reach furthest into their sequences first; of the segments of at_least rows and more
         that have fewer than `below`."""
+        return self.once(("row_tiles", size, at_least, below), lambda: self._row_tiles(size, at_least, below))
+
+    def _row_tiles(self, size: int, at_least: int, below: int) -> tuple[list[Tensor], int]:
         some = np.flatnonzero((self.count >= at_least) & (self.count < below))
         start, count, length = self.first[some], self.count[some], (self.starts + self.count)
         per = (count + size - 1) // size
@@ -123,6 +140,9 @@ class RowPlan:
     def chunks(self, size: int) -> tuple[list[Tensor], int]:
         """([segment's first chunk (n + 1), chunk's first row, chunk's rows, the segment's rows before it], number of chunks) for
         chunks of `size` rows."""
+        return self.once(("chunks", size), lambda: self._chunks(size))
+
+    def _chunks(self, size: int) -> tuple[list[Tensor], int]:
         per = (self.count + size - 1) // size
         base = np.concatenate([[0], np.cumsum(per)]).astype(np.int32)
         within = np.arange(base[-1], dtype=np.int32) - np.repeat(base[:-1], per)
@@ -565,17 +585,16 @@ class LatentAttention:
         space, against attending in latent space (whose kernel reads the cache once per row and head tile)."""
         if not self.expanded:
             return False
-        count, length = plan.count.astype(np.float64), (plan.starts + plan.count).astype(np.float64)
-        pairs = float((count * (length - count / 2)).sum())
-        expanded = float(length.sum()) * self.rank * (self.dim + self.vdim) + pairs * (self.dim + self.rot + self.vdim)
+        positions, _, pairs = plan.extent()
+        expanded = float(positions) * self.rank * (self.dim + self.vdim) + pairs * (self.dim + self.rot + self.vdim)
         return expanded < 2.0 * pairs * (2 * self.rank + self.rot)
 
     def run_expanded(self, a: Latent, rows: Rows, out: Tensor) -> None:
         plan, lib, bf = rows.plan, cuda_library("latent_attn"), torch.bfloat16
-        n_ctx = int((plan.starts + plan.count).sum())
+        n_ctx, longest, _ = plan.extent()
         slots, first = plan.contexts()
         N, K = self.w_ukv.shape
-        a.rotate_q, a.max_len, a.n_contexts = 1, int((plan.starts + plan.count).max()), plan.n_segments
+        a.rotate_q, a.max_len, a.n_contexts = 1, longest, plan.n_segments
         a.ctx_slot, a.ctx_first = slots.data_ptr(), first.data_ptr()
         a.ctx_ld, a.ctx_kv_ld = K, N
         a.ctx = rows.buffer("latent_ctx", n_ctx * K, bf, self.device).data_ptr()

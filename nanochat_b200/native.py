@@ -252,7 +252,7 @@ def stream() -> ctypes.c_void_p:
     more host time than small passes spend on the device.)"""
     import torch
 
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def check(status: int, what: str) -> None:
