@@ -550,7 +550,8 @@ int short_conv_tail(const ncb_conv *args, int f32, int *status, void *stream);
  *   gqa_merge    out [rows][ldo] = sigmoid(gate) * merged states
  *   gqa_prefill  out of row tiles, bf16: tile_rows (at most 64) rows from tile_row, the first at position tile_pos. List the
  *                tiles that reach furthest first. For gqa_prefill_supported(dim, vdim)
- *   gqa_prefill_tiles  the same with at most 128 rows per tile, for gqa_prefill_tiles_supported sizes; scale positive, ldo a multiple of 8 */
+ *   gqa_prefill_tiles  the same with at most 128 rows per tile, for gqa_prefill_tiles_supported sizes; scale positive, ldo a multiple of 8
+ *   gqa_prefill_f32    the same with at most 8 rows per tile, everything fp32, for gqa_prefill_f32_supported sizes */
 #define NCB_GQA_TILE 16
 typedef struct {
     ncb_conv conv;
@@ -573,6 +574,8 @@ int gqa_prefill_supported(int dim, int vdim);
 int gqa_prefill(const ncb_gqa *args, void *stream);
 int gqa_prefill_tiles_supported(int dim, int vdim);
 int gqa_prefill_tiles(const ncb_gqa *args, void *stream);
+int gqa_prefill_f32_supported(int dim, int vdim);
+int gqa_prefill_f32(const ncb_gqa *args, void *stream);
 
 /* ---- library delta_rule ------------------------------------------------------------------------------------------------
  * Gated delta rule with a decay per key channel (csrc/delta_rule.cu has the recurrence). T as above. Projected rows hold q, k

@@ -10,6 +10,7 @@
  *     mma.sync.m16n8k16. Every warp walks its own 16-position tiles, whose rows come by bulk copies into its own ring, with a
  *     softmax state of its own; the block merges its four. In a decode step it also does what k_gqa_rows does: the copies of
  *     the older positions start before the dependency wait, and the new row goes to the cache and straight to its tile;
+ *   - k_gqa_prefill_f32: eight of a prompt's rows against its keys and values in plain fp32 arithmetic, for T = float;
  *   - k_gqa_merge: the chunks' un-normalised states (m in log2 units, l, o) and the gate;
  *   - k_gqa_prefill_tiles: a tile of a prompt's rows of one query head against the cached keys and values on tcgen05, for heads of 64 and
  *     128; k_gqa_prefill: the same on mma.sync, for other sizes and for short segments.
@@ -741,6 +742,118 @@ template <int KB, int VB> __global__ void __launch_bounds__(att::BOUND, 2) k_gqa
         });
 }
 
+/* ---- prompts in 32 bits ------------------------------------------------------------------------------------------------ */
+
+constexpr int F32_ROWS = 8, F32_KEYS = 32;
+
+/* Floats of shared memory of k_gqa_prefill_f32: queries, two stages of keys (rows padded by 4) and values, probabilities [key][row]. */
+__host__ __device__ inline int f32_smem(int dim, int vdim) { return F32_ROWS * dim + 2 * F32_KEYS * (dim + 4 + vdim) + F32_KEYS * F32_ROWS; }
+
+/* Grid (heads, row tiles): at most 8 consecutive rows of a sequence against its keys, 32 at a time, everything in fp32. k_gqa_split_any
+ * reads all keys and values from L2 for every row (bound by that: 2.8 TB/s); here eight rows share them. Scores: a lane has a key, a
+ * warp two rows. Values: a thread has NV columns of all rows. One sequence of 300 rows, 6 heads of 128, split and merge -> this:
+ * 108 -> 45 us a layer. */
+template <int NV> __global__ void __launch_bounds__(THREADS) k_gqa_prefill_f32(const ncb_gqa a) {
+    extern __shared__ __align__(16) float shared[];
+    __shared__ float shrink[F32_ROWS], sums[F32_ROWS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.x, tile = blockIdx.y, W = a.dim + a.vdim, ks = a.dim + 4;
+    float *q = shared, *k = q + F32_ROWS * a.dim, *v = k + 2 * F32_KEYS * ks, *p = v + 2 * F32_KEYS * a.vdim;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int row0 = a.tile_row[tile], rows = min(a.tile_rows[tile], F32_ROWS), pos0 = a.tile_pos[tile];
+    int slot = 0, end;
+    const bool ok = rows > 0 && length_of(a, row0, slot) > 0 && length_of(a, row0 + rows - 1, end) == pos0 + rows; /* flagged by gqa_rows too */
+    float *out = (float *)a.out + (size_t)row0 * a.ldo + h * a.vdim;
+    if (!ok) {
+        for (int i = tid; i < rows * a.vdim; i += THREADS) out[(size_t)(i / a.vdim) * a.ldo + i % a.vdim] = 0.f;
+        return;
+    }
+    const float *cache = cache_row<float>(a, slot, h / (a.heads / a.kv_heads), 0);
+    const int keys = pos0 + rows, n = (keys + F32_KEYS - 1) / F32_KEYS;
+    auto fetch = [&](int i) { /* positions past the tile's last row are zeros */
+        float *kd = k + (i & 1) * F32_KEYS * ks, *vd = v + (i & 1) * F32_KEYS * a.vdim;
+        const int per = W / 4;
+        for (int c = tid; c < F32_KEYS * per; c += THREADS) {
+            const int j = c / per, at = c % per * 4, key = i * F32_KEYS + j;
+            cp_async16(smem_u32(at < a.dim ? kd + j * ks + at : vd + j * a.vdim + at - a.dim), cache + (size_t)min(key, keys - 1) * W + at, key < keys);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    for (int i = tid; i < F32_ROWS * a.dim; i += THREADS)
+        q[i] = i / a.dim < rows ? ((const float *)a.q)[((size_t)(row0 + i / a.dim) * a.heads + h) * a.dim + i % a.dim] : 0.f;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[NV][F32_ROWS];
+#pragma unroll
+    for (int c = 0; c < NV; c++)
+#pragma unroll
+        for (int r = 0; r < F32_ROWS; r++) acc[c][r] = 0.f;
+    const float scale = a.scale * LOG2E;
+    for (int i = 0; i < n; i++) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads(); /* this stage is there, and all are done with the other */
+        if (i + 1 < n) fetch(i + 1);
+        const int key = i * F32_KEYS + lane;
+        {
+            const float *kr = k + (i & 1) * F32_KEYS * ks + lane * ks, *q0 = q + 2 * warp * a.dim, *q1 = q0 + a.dim;
+            float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+#pragma unroll 4
+            for (int d = 0; d < a.dim; d += 4) {
+                const float4 x = *reinterpret_cast<const float4 *>(kr + d), y = *reinterpret_cast<const float4 *>(q0 + d), z = *reinterpret_cast<const float4 *>(q1 + d);
+                s0.x = fmaf(x.x, y.x, s0.x), s0.y = fmaf(x.y, y.y, s0.y), s0.z = fmaf(x.z, y.z, s0.z), s0.w = fmaf(x.w, y.w, s0.w);
+                s1.x = fmaf(x.x, z.x, s1.x), s1.y = fmaf(x.y, z.y, s1.y), s1.z = fmaf(x.z, z.z, s1.z), s1.w = fmaf(x.w, z.w, s1.w);
+            }
+            const float dots[2] = {(s0.x + s0.y) + (s0.z + s0.w), (s1.x + s1.y) + (s1.z + s1.w)};
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int r = 2 * warp + e;
+                const float s = key <= pos0 + r && r < rows ? dots[e] * scale : -INFINITY;
+                float top = s;
+                for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+                const float next = fmaxf(m[e], top), x = r < rows ? exp2f(s - next) : 0.f, f = r < rows ? exp2f(m[e] - next) : 0.f;
+                float sum = x;
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                l[e] = l[e] * f + sum;
+                m[e] = next;
+                p[lane * F32_ROWS + r] = x;
+                if (lane == 0) shrink[r] = f;
+            }
+        }
+        __syncthreads();
+        const float *vs = v + (i & 1) * F32_KEYS * a.vdim;
+        const int all = min(max(pos0 + 1 - i * F32_KEYS, 0), F32_KEYS), some = min(keys - i * F32_KEYS, F32_KEYS); /* keys that every row, some row sees */
+#pragma unroll
+        for (int c = 0; c < NV; c++) {
+            const int col = tid + c * THREADS;
+            if (col >= a.vdim) continue;
+#pragma unroll
+            for (int r = 0; r < F32_ROWS; r++) acc[c][r] *= shrink[r];
+#pragma unroll 4
+            for (int j = 0; j < all; j++) {
+                const float x = vs[j * a.vdim + col];
+                const float4 lo = *reinterpret_cast<const float4 *>(p + j * F32_ROWS), hi = *reinterpret_cast<const float4 *>(p + j * F32_ROWS + 4);
+                acc[c][0] = fmaf(lo.x, x, acc[c][0]), acc[c][1] = fmaf(lo.y, x, acc[c][1]), acc[c][2] = fmaf(lo.z, x, acc[c][2]), acc[c][3] = fmaf(lo.w, x, acc[c][3]);
+                acc[c][4] = fmaf(hi.x, x, acc[c][4]), acc[c][5] = fmaf(hi.y, x, acc[c][5]), acc[c][6] = fmaf(hi.z, x, acc[c][6]), acc[c][7] = fmaf(hi.w, x, acc[c][7]);
+            }
+            for (int j = all; j < some; j++) { /* a value that is not finite must not reach a row that does not see it, not even times zero */
+                const float x = vs[j * a.vdim + col];
+#pragma unroll
+                for (int r = 0; r < F32_ROWS; r++)
+                    if (i * F32_KEYS + j <= pos0 + r) acc[c][r] = fmaf(p[j * F32_ROWS + r], x, acc[c][r]);
+            }
+        }
+    }
+    if (lane == 0) sums[2 * warp] = l[0], sums[2 * warp + 1] = l[1];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < F32_ROWS; r++)
+        if (r < rows) {
+            const float z = ((const float *)a.conv.proj)[(size_t)(row0 + r) * a.conv.ldp + a.off_g + h], f = 1.f / ((1.f + expf(-z)) * sums[r]);
+#pragma unroll
+            for (int c = 0; c < NV; c++)
+                if (tid + c * THREADS < a.vdim) out[(size_t)r * a.ldo + tid + c * THREADS] = acc[c][r] * f;
+        }
+}
+
 /* ---- merge and gate --------------------------------------------------------------------------------------------------- */
 
 /* Grid (heads, rows): the chunks' states of a head, its gate. */
@@ -878,6 +991,22 @@ int gqa_prefill(const ncb_gqa *g, void *stream) {
     if (g->dim == 64 && g->vdim == 64) return launch(k_gqa_prefill<4, 4, true>, grid, THREADS, smem, 1, s, *g);
     return g->dim <= 128 ? launch(k_gqa_prefill<8, 8, false>, grid, THREADS, smem, 1, s, *g)
                          : launch(k_gqa_prefill<12, 8, false>, grid, THREADS, smem, 1, s, *g);
+}
+
+/* 1 if gqa_prefill_f32 takes these (padded) sizes. */
+int gqa_prefill_f32_supported(int dim, int vdim) { return dim > 0 && vdim > 0 && dim % 16 == 0 && vdim % 16 == 0 && vdim <= 2 * THREADS && (size_t)f32_smem(dim, vdim) * 4 <= 200 * 1024; }
+
+int gqa_prefill_f32(const ncb_gqa *g, void *stream) {
+    if (!g) return NCB_ERR_ARG;
+    const int rc = check(*g);
+    if (rc != NCB_OK || g->conv.rows == 0 || g->n_tiles == 0) return rc;
+    if (!gqa_prefill_f32_supported(g->dim, g->vdim)) return NCB_ERR_UNSUPPORTED;
+    if (!g->q || !g->out || g->ldo < g->heads * g->vdim || !g->tile_row || !g->tile_rows || !g->tile_pos || g->n_tiles < 0 || g->n_tiles > 65535)
+        return NCB_ERR_ARG;
+    const dim3 grid(g->heads, g->n_tiles);
+    const size_t smem = (size_t)f32_smem(g->dim, g->vdim) * 4;
+    return g->vdim <= THREADS ? launch(k_gqa_prefill_f32<1>, grid, THREADS, smem, 1, (cudaStream_t)stream, *g)
+                              : launch(k_gqa_prefill_f32<2>, grid, THREADS, smem, 1, (cudaStream_t)stream, *g);
 }
 
 /* 1 if gqa_prefill_tiles takes these (padded) sizes. */

@@ -264,9 +264,11 @@ class GroupedAttention:
         self.fused = bf and bool(lib.gqa_split_fused(self.dim, self.vdim))
         self.tiled = bf and bool(lib.gqa_prefill_supported(self.dim, self.vdim))
         self.wide = self.tiled and self.scale > 0.0 and bool(lib.gqa_prefill_tiles_supported(self.dim, self.vdim))
+        self.tiled_f32 = not bf and bool(lib.gqa_prefill_f32_supported(self.dim, self.vdim))
 
     ROW_TILE = 64     # rows per tile of gqa_prefill
     WIDE_TILE = 128   # rows per tile of gqa_prefill_tiles
+    F32_TILE = 8      # rows per tile of gqa_prefill_f32
     TILED_FROM = 8    # shorter segments run as rows on their own
     # Segments from which gqa_prefill_tiles (tcgen05) has them, beside shorter ones of the pass. 10 heads of 128, us, gqa_prefill -> gqa_prefill_tiles: sixteen segments of
     # 16 rows 11.3 -> 13.3, of 32 13.3 -> 13.3, of 100 21 -> 17; eight of 511 48 -> 28; one of 4,088 229 -> 105 (16 heads over 4: 335 -> 116).
@@ -331,6 +333,11 @@ class GroupedAttention:
                 a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
                 entry = "gqa_prefill_tiles" if wide else "gqa_prefill"
                 check(getattr(lib, entry)(pointer_to(a), stream()), entry)
+        elif (out is not None and self.tiled_f32 and rows.plan is not None and rows.plan.longest >= self.TILED_FROM
+              and rows.plan.row_tiles(self.F32_TILE)[1] <= 65535):
+            tiles, a.n_tiles = rows.plan.row_tiles(self.F32_TILE)
+            a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+            check(lib.gqa_prefill_f32(pointer_to(a), stream()), "gqa_prefill_f32")
         elif out is not None:
             max_len = min(rows.max_len, kv.capacity)
             tiles = (max_len + GQA_TILE - 1) // GQA_TILE

@@ -167,6 +167,8 @@ SIGNATURES = {
         "gqa_prefill": ([c_ptr, c_ptr], c_int),
         "gqa_prefill_tiles_supported": ([c_int] * 2, c_int),
         "gqa_prefill_tiles": ([c_ptr, c_ptr], c_int),
+        "gqa_prefill_f32_supported": ([c_int] * 2, c_int),
+        "gqa_prefill_f32": ([c_ptr, c_ptr], c_int),
     },
     "delta_rule": {
         "delta_step": ([c_ptr, c_int, c_ptr], c_int),

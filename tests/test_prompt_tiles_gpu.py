@@ -346,3 +346,44 @@ def test_a_segments_length_chooses_its_kernel(kind):
     for n in counts:
         assert torch.equal(together[row:row + n], run_counts(mixer, [n], proj[row:row + n])), n
         row += n
+
+
+@pytest.mark.parametrize("runs", [[(0, 1)], [(0, 8), (3, 9)], [(31, 7), (32, 16), (25, 8)], [(300, 45), (0, 130)]], ids=str)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 4, 128, 128), (6, 2, 16, 48), (2, 1, 80, 256)])
+def test_grouped_in_32_bits(heads, kv_heads, dim, vdim, runs):
+    """gqa_prefill_f32 around the edges of its tiles of 8 rows and 32 keys, with NaN behind each sequence's end and infinities in the values
+    of its last position, against float64: a sum of at most 345 weighted values and 128 products per score, a few times sqrt(345) 2^-24
+    of the result's size; infinities only where the last position is seen."""
+    gen = torch.Generator(device="cuda").manual_seed(75)
+    slots, pos = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
+    n, capacity, scale = len(pos), 384, dim ** -0.5
+    ldp = heads * dim  # the projection's rows: only the gate is read
+    q, proj = torch.randn(n, heads, dim, generator=gen, device="cuda"), torch.randn(n, ldp, generator=gen, device="cuda")
+    gate = proj[:, :heads]
+    kv = torch.full((len(runs), kv_heads, capacity, dim + vdim), float("nan"), device="cuda")
+    for s, (at, count) in enumerate(runs):
+        kv[s, :, :at + count] = torch.randn(kv_heads, at + count, dim + vdim, generator=gen, device="cuda")
+        if at + count > 1:
+            kv[s, :, at + count - 1, dim:] = float("inf")
+    dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slots)]
+    status, plan, lib = torch.zeros(1, dtype=torch.int32, device="cuda"), RowPlan(slots, pos, "cuda"), cuda_library("gqa_attn")
+    ring, taps = torch.zeros(len(runs), 1, ldp, device="cuda"), torch.ones(1, ldp, device="cuda")
+    out = torch.full((n, heads * vdim + 8), 7.0, device="cuda")
+    a = Gqa(conv=Conv(proj=proj.data_ptr(), ring=ring.data_ptr(), w=taps.data_ptr(), rows=n, ldp=ldp, taps=1, width=ldp, n_slots=len(runs),
+                      pos=dev[0].data_ptr(), slot_map=dev[1].data_ptr()), q=q.data_ptr(), kv=kv.data_ptr(), out=out.data_ptr(), ldo=out.stride(0),
+            heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, norm_count=dim, capacity=capacity, table_len=capacity, scale=scale, eps=1e-6,
+            status=status.data_ptr())
+    tiles, a.n_tiles = plan.row_tiles(8)
+    a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+    check(lib.gqa_prefill_f32(ctypes.byref(a), stream()), "gqa_prefill_f32")
+    assert int(status.item()) == 0 and bool((out[:, heads * vdim:] == 7.0).all())
+    got, row = out[:, :heads * vdim].view(n, heads, vdim), 0
+    for s, (at, count) in enumerate(runs):
+        k, v = (t.repeat_interleave(heads // kv_heads, 0) for t in kv[s, :, :at + count].split([dim, vdim], -1))
+        seen = count - 1 if at + count > 1 else count  # rows that do not see the infinite values
+        if seen:
+            want = attended(q[row:row + seen], k[:, :at + seen], v[:, :at + seen], scale, at) * torch.sigmoid(gate[row:row + seen].to(F64))[..., None]
+            assert float((got[row:row + seen].to(F64) - want).abs().max() / want.abs().max()) < 5e-6
+        if seen < count:
+            assert not torch.isfinite(got[row + count - 1]).any()
+        row += count
