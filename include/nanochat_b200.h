@@ -173,7 +173,8 @@ long long decode_attn_workspace_bytes(int B, int Hq, int max_kv_len, int Hkv, in
  * Two launches: the split-KV kernel (one block per sequence, kv head and chunk of pages; all Hq/Hkv query heads
  * of the kv head share each K/V byte) and the merge kernel. When max_kv_len and chunk_pages leave every sequence one
  * chunk (at most four pages of cache, or a chunk size of at least the cache's pages) the split kernel's blocks
- * normalise and write `out` themselves and there is no second launch; the output bits are the same either way.
+ * normalise and write `out` themselves and there is no second launch, and with two to eight chunks in a grid that fits the
+ * GPU at once a sequence's blocks are a cluster that merges its states itself; the output bits are the same either way.
  */
 int decode_attn_fp8(const void *q, const void *kv_cache, const void *lens, const void *slot_map, void *workspace,
                     long long workspace_bytes, void *out, int B, int Hq, int Hkv, int n_slots, int pages_per_slot,
@@ -190,7 +191,7 @@ int decode_attn_fp8_partial(const void *q, const void *kv_cache, const void *len
                             float softmax_scale, void *status, void *stream);
 
 /*
- * kv_append_fp8 and decode_attn_fp8 for one new token per sequence in the same two launches as decode_attn_fp8
+ * kv_append_fp8 and decode_attn_fp8 for one new token per sequence in the same launches as decode_attn_fp8
  * alone (replaces k_prologue + k_attn, decode.cu:859-863, as a pair): every block of the split-KV kernel first does
  * the append's arithmetic for its own heads — q rows stay in shared memory, the block whose chunk holds the new
  * position writes that kv head's k and v bytes and scales into the cache — and then attends over positions

@@ -219,10 +219,10 @@ class PrefillPlan:
     # meets enough pairs (a row and a position it attends): WIDE_PAIRS, and with all query heads of a key/value head WIDE_GROUP_PAIRS.
     # From position 0 that is 384 rows where every query head has its own key/value head, else 192. Measured, append and attention of
     # whole prompts, heads over key/value heads, us, prefill_attn_fp8 -> tiles:
-    #   10 / 10   1 x 256  21.0 -> 16.5   8 x 256 31.6 -> 32.4   8 x 512 56.9 -> 55.8   16 x 100 24.8 -> 33.3    1 x 4096 243 -> 130
-    #   16 / 16   1 x 256  22.0 -> 18.8   8 x 256 39.6 -> 46.0   8 x 512 92.1 -> 80.7   16 x 100 34.9 -> 43.5    1 x 4096 337 -> 154
-    #   32 / 8    1 x 256  24.8 -> 17.9   8 x 256 56.0 -> 49.5   8 x 512 142 -> 98      16 x 100 39.9 -> 42.6    1 x 4096 625 -> 235
-    #   16 / 2    1 x 256  21.1 -> 15.1   8 x 256 30.3 -> 27.8   8 x 512 71.0 -> 50.2   16 x 100 21.2 -> 24.6    1 x 4096 317 -> 134
+    #   10 / 10   1 x 256  21.1 -> 17.6   8 x 256 31.1 -> 34.8   8 x 512 53.4 -> 54.2   16 x 100 21.8 -> 30.4    1 x 4096 241 -> 122
+    #   16 / 16   1 x 256  22.1 -> 18.3   8 x 256 35.9 -> 43.3   8 x 512 84.0 -> 75.6   16 x 100 30.0 -> 36.9    1 x 4096 331 -> 142
+    #   32 / 8    1 x 256  23.2 -> 17.3   8 x 256 52.4 -> 51.0   8 x 512 137 -> 100     16 x 100 36.6 -> 42.5    1 x 4096 621 -> 230
+    #   16 / 2    1 x 256  21.8 -> 16.4   8 x 256 29.6 -> 27.5   8 x 512 69.2 -> 48.9   16 x 100 19.9 -> 24.7    1 x 4096 317 -> 116
     # (A single prompt of 256 to 383 rows with equal heads would gain, eight of them would lose, and a row's kernel must not depend on
     # the others.)
     WIDE_ROWS = 64                # rows of a portion
