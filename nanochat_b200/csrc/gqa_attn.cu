@@ -365,8 +365,11 @@ __host__ __device__ inline SplitSmem split_smem(int dim, int vdim, int stages) {
     return s;
 }
 
-/* Grid (max chunks, kv_heads x tiles of 16 query heads, rows). DK, VN: upper bounds of dim / 16 and vdim / 16. */
-template <int DK, int VN> __global__ void __launch_bounds__(THREADS, DK + VN > 16 ? 1 : 2) k_gqa_split(const ncb_gqa a, int stages) {
+/* Grid (max chunks, kv_heads x tiles of 16 query heads, rows). DK, VN: upper bounds of dim / 16 and vdim / 16. UPPER: a block has more than
+ * eight heads; else the upper half of the MMAs' rows is zero and nothing is computed for it, which leaves registers for three blocks per
+ * SM: every warp waits on its own chain of products and exponentials, so more warps are what helps. 16 heads over 4, batch 32 of 256 to
+ * 8,192 positions, 16 layers: a step 2,948 -> 2,742 us (without the upper half alone 2,948). */
+template <int DK, int VN, bool UPPER> __global__ void __launch_bounds__(THREADS, DK + VN > 16 ? 1 : UPPER ? 2 : 3) k_gqa_split(const ncb_gqa a, int stages) {
     extern __shared__ __align__(128) uint8_t raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, row = blockIdx.z;
     const int R = a.heads / a.kv_heads, head_tiles = (R + HEADS_M - 1) / HEADS_M, kvh = blockIdx.y / head_tiles;
@@ -475,25 +478,33 @@ template <int DK, int VN> __global__ void __launch_bounds__(THREADS, DK + VN > 1
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const bool on = n * 8 + 2 * t + e < live;
-                p[n][e] = on ? p[n][e] * scale : -INFINITY, p[n][2 + e] = on ? p[n][2 + e] * scale : -INFINITY;
-                mx_lo = fmaxf(mx_lo, p[n][e]), mx_hi = fmaxf(mx_hi, p[n][2 + e]);
+                p[n][e] = on ? p[n][e] * scale : -INFINITY;
+                mx_lo = fmaxf(mx_lo, p[n][e]);
+                if (UPPER) p[n][2 + e] = on ? p[n][2 + e] * scale : -INFINITY, mx_hi = fmaxf(mx_hi, p[n][2 + e]);
             }
         mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 1));
-        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
+        if (UPPER) mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
         mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
-        mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-        if (__any_sync(0xffffffffu, mx_lo != m_lo || mx_hi != m_hi)) {
-            const float al = ex2(m_lo - mx_lo), ah = ex2(m_hi - mx_hi); /* 0 for the first tile */
+        if (UPPER) mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
+        if (__any_sync(0xffffffffu, mx_lo != m_lo || (UPPER && mx_hi != m_hi))) {
+            const float al = ex2(m_lo - mx_lo), ah = UPPER ? ex2(m_hi - mx_hi) : 0.f; /* 0 for the first tile */
             l_lo *= al, l_hi *= ah;
 #pragma unroll
             for (int c = 0; c < VN; c++)
 #pragma unroll
-                for (int n = 0; n < 2; n++) o[c][n][0] *= al, o[c][n][1] *= al, o[c][n][2] *= ah, o[c][n][3] *= ah;
+                for (int n = 0; n < 2; n++) {
+                    o[c][n][0] *= al, o[c][n][1] *= al;
+                    if (UPPER) o[c][n][2] *= ah, o[c][n][3] *= ah;
+                }
             m_lo = mx_lo, m_hi = mx_hi;
         }
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int e = 0; e < 4; e++) { /* e: heads g / g + 8, positions 2 t, + 1 / + 8, + 9 */
+            if (!UPPER && (e & 1)) {
+                hi[e] = lo[e] = 0u;
+                continue;
+            }
             const float m = (e & 1) ? m_hi : m_lo;
             const float a0 = ex2(p[e >> 1][2 * (e & 1)] - m), a1 = ex2(p[e >> 1][2 * (e & 1) + 1] - m);
             if (e & 1) l_hi += a0 + a1;
@@ -516,15 +527,14 @@ template <int DK, int VN> __global__ void __launch_bounds__(THREADS, DK + VN > 1
     }
     if (!ok && lane == 0) flag(a.status, NCB_DEV_WAIT_TIMEOUT);
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+    if (UPPER) l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1), l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
     __syncthreads(); /* every ring has been consumed: the warps' states take its place */
     const int state = a.vdim + STATE_PAD;
     float *mine = reinterpret_cast<float *>(raw) + warp * HEADS_M * state;
     if (t == 0) {
         mine[g * state] = m_lo, mine[g * state + 1] = l_lo;
-        mine[(g + 8) * state] = m_hi, mine[(g + 8) * state + 1] = l_hi;
+        if (UPPER) mine[(g + 8) * state] = m_hi, mine[(g + 8) * state + 1] = l_hi;
     }
 #pragma unroll
     for (int c = 0; c < VN; c++)
@@ -533,7 +543,7 @@ template <int DK, int VN> __global__ void __launch_bounds__(THREADS, DK + VN > 1
             for (int n = 0; n < 2; n++) {
                 const int col = STATE_PAD + c * 16 + n * 8 + 2 * t;
                 *reinterpret_cast<float2 *>(mine + g * state + col) = make_float2(o[c][n][0], o[c][n][1]);
-                *reinterpret_cast<float2 *>(mine + (g + 8) * state + col) = make_float2(o[c][n][2], o[c][n][3]);
+                if (UPPER) *reinterpret_cast<float2 *>(mine + (g + 8) * state + col) = make_float2(o[c][n][2], o[c][n][3]);
             }
     __syncthreads();
     for (int h = warp; h < n_heads; h += WARPS) { /* (the chunk's first tile is never empty: some m is finite) */
@@ -939,6 +949,9 @@ int gqa_rows(const ncb_gqa *g, int f32, void *stream) {
 /* 1 if gqa_split in bf16 takes these (padded) sizes with q NULL. */
 int gqa_split_fused(int dim, int vdim) { return dim > 0 && vdim > 0 && dim <= 256 && vdim <= 256; }
 
+/* Blocks of the fused form per SM, as far as registers go (see k_gqa_split): what a plan of chunks may count on. */
+int gqa_split_blocks(int heads, int kv_heads, int dim, int vdim) { return heads / kv_heads <= 8 && dim <= 128 && vdim <= 128 ? 3 : 2; }
+
 int gqa_split(const ncb_gqa *g, int f32, void *stream) {
     if (!g) return NCB_ERR_ARG;
     int rc = check(*g);
@@ -946,13 +959,16 @@ int gqa_split(const ncb_gqa *g, int f32, void *stream) {
     if ((rc = check_parts(*g)) != NCB_OK) return rc;
     if (!f32 && gqa_split_fused(g->dim, g->vdim)) {
         int stages = 4;
-        while (stages > 2 && split_smem(g->dim, g->vdim, stages).total > 112 * 1024) stages--;
+        const bool three = gqa_split_blocks(g->heads, g->kv_heads, g->dim, g->vdim) == 3;
+        while (stages > 2 && split_smem(g->dim, g->vdim, stages).total > (three ? 75 : 112) * 1024) stages--;
         const size_t smem = split_smem(g->dim, g->vdim, stages).total;
         const dim3 grid(g->max_chunks, g->kv_heads * ((g->heads / g->kv_heads + HEADS_M - 1) / HEADS_M), (unsigned)g->conv.rows);
         const cudaStream_t s = (cudaStream_t)stream;
-        if (g->dim <= 64 && g->vdim <= 64) return launch(k_gqa_split<4, 4>, grid, THREADS, smem, 1, s, *g, stages);
-        if (g->dim <= 128 && g->vdim <= 128) return launch(k_gqa_split<8, 8>, grid, THREADS, smem, 1, s, *g, stages);
-        return launch(k_gqa_split<16, 16>, grid, THREADS, smem, 1, s, *g, stages);
+        auto run = [&](auto kernel) { return launch(kernel, grid, THREADS, smem, 1, s, *g, stages); };
+        const bool upper = g->heads / g->kv_heads > 8;
+        if (g->dim <= 64 && g->vdim <= 64) return upper ? run(k_gqa_split<4, 4, true>) : run(k_gqa_split<4, 4, false>);
+        if (g->dim <= 128 && g->vdim <= 128) return upper ? run(k_gqa_split<8, 8, true>) : run(k_gqa_split<8, 8, false>);
+        return upper ? run(k_gqa_split<16, 16, true>) : run(k_gqa_split<16, 16, false>);
     }
     if (!g->q) return NCB_ERR_ARG; /* only the form above prepares its rows */
     const size_t smem = (size_t)(g->dim + g->vdim + ANY_TILE + 8) * 4;

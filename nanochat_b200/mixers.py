@@ -294,15 +294,16 @@ class GroupedAttention:
 
     def chunk_for(self, lens: "list[int]", most: int) -> int:
         """Tiles per chunk of the split kernel for rows of these lengths, at most 128 chunks for `most` positions: enough blocks
-        to fill the GPU twice over, chunks long enough to be worth a state."""
+        to fill the GPU (gqa_split_blocks per SM), chunks long enough to be worth a state."""
         tiles = np.maximum((np.asarray(lens, dtype=np.int64) + GQA_TILE - 1) // GQA_TILE, 1)
         top, least = int(tiles.max()), max(8, ((most + GQA_TILE - 1) // GQA_TILE + 127) // 128)
         per_chunk = self.kv_heads * ((self.heads // self.kv_heads + 15) // 16)
+        places = SM_COUNT * cuda_library("gqa_attn").gqa_split_blocks(self.heads, self.kv_heads, self.dim, self.vdim)
         best, cost = least, float("inf")
         c = least
         while c < 2 * max(top, least):
             blocks = int(((tiles + c - 1) // c).sum()) * per_chunk
-            now = -(-blocks // (2 * SM_COUNT)) * (min(c, top) + 8.0)
+            now = -(-blocks // places) * (min(c, top) + 8.0)
             if now < cost:
                 best, cost = c, now
             c += max(1, c // 8)

@@ -163,6 +163,7 @@ SIGNATURES = {
         "gqa_split": ([c_ptr, c_int, c_ptr], c_int),
         "gqa_merge": ([c_ptr, c_int, c_ptr], c_int),
         "gqa_split_fused": ([c_int] * 2, c_int),
+        "gqa_split_blocks": ([c_int] * 4, c_int),
         "gqa_prefill_supported": ([c_int] * 2, c_int),
         "gqa_prefill": ([c_ptr, c_ptr], c_int),
         "gqa_prefill_tiles_supported": ([c_int] * 2, c_int),
