@@ -332,7 +332,8 @@ static __device__ __forceinline__ void query_fragments(const float *q_stage, con
 
 /* The chunks of a sequence and key/value head are the blocks of one cluster; each left its state of every head at `own` [S][PART] in its
  * shared memory; out [S][128]. Chunk c folds and normalises heads c, c + the number of chunks, ..: thread = dimension, k_merge's arithmetic in
- * k_merge's order (four runs of every fourth state, then the runs), so the bits are the same. Blocks without pages have left. */
+ * k_merge's order (four runs of every fourth state, then the runs), so the bits are the same. Blocks without pages have left. `chunks` never
+ * exceeds the cluster: a sequence longer than the caller's bound has more chunks than there are blocks, and is cut off as in k_merge. */
 static __device__ __noinline__ void join_chunks(bf16 *out, float *own, int chunks, int chunk, int S, int tid) {
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync(); /* every state is there */
@@ -580,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS_PER_SM) k_decode_attn(AttnArgs
     }
     if (a.joined)
         join_chunks(a.direct + ((size_t)b * a.Hq + (size_t)kvh * G) * HEAD_DIM, merge + WARPS * 4 * NT * PART,
-                    (sp.last_page - sp.first_page + sp.chunk - 1) / sp.chunk /* that have pages */, chunk, S, tid);
+                    min(sp.n_chunks, a.max_chunks), chunk, S, tid);
 }
 
 /* ---- prefill attention --------------------------------------------------------------------------------------- */

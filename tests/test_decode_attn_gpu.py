@@ -493,3 +493,21 @@ def test_chunks_that_join_in_a_cluster_give_the_merge_launch_s_bits(heads, kv_he
     part = ncb.decode_attention_partial(q, cache, lens_t, **args)
     want = ncb.merge_partials(part[None].contiguous())
     assert torch.equal(out, want) and not out[4:].any() and bool(out[:4].any())
+
+
+@pytest.mark.parametrize("window", [0, 700])
+@pytest.mark.parametrize("chunk_pages,bound", [(4, 512), (2, 300), (1, 130), (3, 1)])
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (8, 2), (16, 2)])
+def test_sequences_longer_than_the_bound_are_cut_off_alike_by_cluster_and_merge_launch(heads, kv_heads, chunk_pages, bound, window):
+    """A length above max_kv_len and inside the cache has more chunks than blocks: a row cut off, the same bits from both merges, and
+    every head of it written; rows within the bound are whole."""
+    lens = [bound, bound + 1, 513, 950, 1]
+    case = helpers.attention_case(960 + heads + chunk_pages, heads, kv_heads, lens)
+    cache, q = load_cache(case, max(lens)), helpers.bits_bf16(case["q"]).cuda()
+    lens_t = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    args = dict(max_kv_len=bound, window=window, chunk_pages=chunk_pages)
+    out = torch.full(q.shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    ncb.decode_attention(q, cache, lens_t, out=out, **args)
+    want = ncb.merge_partials(ncb.decode_attention_partial(q, cache, lens_t, **args)[None].contiguous())
+    whole = ncb.decode_attention(q, cache, lens_t, max_kv_len=max(lens), window=window, chunk_pages=chunk_pages)
+    assert torch.equal(out, want) and torch.equal(out[0], whole[0]) and not bool((out == 7.0).all(-1).any())
