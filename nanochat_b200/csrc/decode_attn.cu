@@ -1128,10 +1128,24 @@ struct AppendIn {
     ValueEmbed ve;
 };
 
-/* Whether a launch's chunks join in clusters: see launch_split. One sequence of 512 positions, 10 heads, eager calls: 18.2 -> 15.9 us (one launch
- * instead of two); inside a captured step the same (a d20 step at 8 x 512: 545 us both ways). */
-static bool joins(int max_chunks, int B, int Hkv) {
-    return max_chunks > 1 && max_chunks <= 8 && (long long)max_chunks * B * Hkv <= (long long)BLOCKS_PER_SM * sm_count();
+/* Whether a launch's chunks join in clusters. One launch instead of two is what a host-bound caller gains: one sequence of 512 positions, 10
+ * heads, eager calls one after the other 14.7 -> 13.3 us, 8 x 768 13.7 -> 11.3, 1 x 2,048 in eight chunks 18.4 -> 11.1. Not
+ *   - under capture: a replayed step has no launches to save, and what follows (the output product's weights, the other branches of a graph)
+ *     overlaps the merge launch better than a cluster that holds its SMs to the end. With all of them joined DecodeStep 64 x 8,192 in eight
+ *     branches takes 220 us a step, not 197; nanochat d20 batch 8 from 512 to 768 604, not 574; two chunks of 512 positions 2 to 3 % less or
+ *     more (batch 4 and 8, batch 1);
+ *   - more than two heads for a block to fold: 8 heads over a key/value head in two and three chunks, 64 x 768 16.7 -> 18.1, 3 x 2,048
+ *     15.4 -> 16.1 (four to eight chunks gain as above);
+ *   - grids that do not fit the GPU at once: a cluster would hold its places until its last chunk is done. */
+static bool joins(int max_chunks, int B, int Hq, int Hkv, cudaStream_t stream) {
+    if (max_chunks < 2 || max_chunks > 8 || Hq / Hkv > 2 * max_chunks || (long long)max_chunks * B * Hkv > (long long)BLOCKS_PER_SM * sm_count())
+        return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+        cudaGetLastError(); /* the launch says what is wrong */
+        return false;
+    }
+    return capture == cudaStreamCaptureStatusNone;
 }
 
 template <int NT, bool APPEND> static cudaError_t prepare() { /* opt in to the large dynamic shared memory, once per device */
@@ -1150,7 +1164,8 @@ template <int NT, bool APPEND> static cudaError_t prepare() { /* opt in to the l
 static int launch_split(const void *q, const void *kv_cache, const void *lens, const void *slot_map, void *workspace,
                         long long workspace_bytes, int B, int Hq, int Hkv, int n_slots, int pages_per_slot,
                         int max_kv_len, int window, int &chunk_pages, float softmax_scale, void *status,
-                        cudaStream_t stream, const AppendIn *app = nullptr, bool early = false, void *direct_out = nullptr) {
+                        cudaStream_t stream, const AppendIn *app = nullptr, bool early = false, void *direct_out = nullptr,
+                        bool *finished = nullptr) {
     if (B < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv != 0 || n_slots <= 0 || pages_per_slot <= 0 || max_kv_len < 0 ||
         window < 0 || chunk_pages < 0 || !(softmax_scale > 0.f))
         return NCB_ERR_ARG;
@@ -1188,11 +1203,11 @@ static int launch_split(const void *q, const void *kv_cache, const void *lens, c
         a.qkv_row_stride = app->qkv_row_stride, a.table_len = app->table_len;
         a.ve = app->ve;
     }
-    /* A sequence's sole chunk writes the output itself. So do a few chunks as one cluster, while the grid fits the GPU at once: in larger
-     * ones a cluster would hold its places until its last chunk is done, and a merge launch costs little beside them. */
-    const bool joined = direct_out && joins(max_chunks, B, Hkv);
+    /* A sequence's sole chunk writes the output itself; so do a few chunks as one cluster (joins). */
+    const bool joined = direct_out && joins(max_chunks, B, Hq, Hkv, stream);
     a.direct = max_chunks == 1 || joined ? (bf16 *)direct_out : nullptr;
     a.joined = joined;
+    if (finished) *finished = a.direct != nullptr;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(max_chunks, Hkv, B);
     config.blockDim = dim3(THREADS);
@@ -1276,16 +1291,16 @@ static int attend(const void *q, const void *kv_cache, const void *lens, const v
                   void *stream, const AppendIn *app = nullptr, const ExchangeIn *exchange = nullptr) {
     if (!out && !part_out) return NCB_ERR_ARG;
     if (((uintptr_t)out | (uintptr_t)part_out) % 16 != 0) return NCB_ERR_ALIGN;
-    /* One chunk per sequence (short caches, or a chunk size at least the cache's pages): the split kernel's blocks
-     * normalise and write the output themselves and there is no merge launch (launch_split takes `out` only then). */
+    /* One chunk per sequence (short caches, or a chunk size at least the cache's pages) or a few that join: the split kernel's blocks
+     * normalise and write the output themselves and there is no merge launch. */
     void *direct = (out && !part_out && !exchange) ? out : nullptr;
+    bool finished = false;
     const int rc = launch_split(q, kv_cache, lens, slot_map, workspace, workspace_bytes, B, Hq, Hkv, n_slots,
                                 pages_per_slot, max_kv_len, window, chunk_pages, softmax_scale, status,
-                                (cudaStream_t)stream, app, exchange != nullptr, direct);
-    if (rc != NCB_OK || B == 0) return rc;
+                                (cudaStream_t)stream, app, exchange != nullptr, direct, &finished);
+    if (rc != NCB_OK || B == 0 || finished) return rc;
     if (max_kv_len > pages_per_slot * PAGE_TOKENS) max_kv_len = pages_per_slot * PAGE_TOKENS;
     const int max_chunks = max(1, (pages_of(max_kv_len) + chunk_pages - 1) / chunk_pages);
-    if (direct && (max_chunks == 1 || joins(max_chunks, B, Hkv))) return NCB_OK;
     MergeArgs m = {(const float *)workspace, (long long)B * Hq, PART, (long long)max_chunks * PART, 0,
                    (const int32_t *)lens, (const int32_t *)slot_map, Hq, window, chunk_pages, n_slots, pages_per_slot,
                    max_chunks, app ? 1 : 0, (bf16 *)out, (float *)part_out, app ? app->table_len : 0};

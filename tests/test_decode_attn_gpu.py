@@ -511,3 +511,27 @@ def test_sequences_longer_than_the_bound_are_cut_off_alike_by_cluster_and_merge_
     want = ncb.merge_partials(ncb.decode_attention_partial(q, cache, lens_t, **args)[None].contiguous())
     whole = ncb.decode_attention(q, cache, lens_t, max_kv_len=max(lens), window=window, chunk_pages=chunk_pages)
     assert torch.equal(out, want) and torch.equal(out[0], whole[0]) and not bool((out == 7.0).all(-1).any())
+
+
+@pytest.mark.parametrize("heads,kv_heads,chunk_pages,joined", [(10, 10, 4, True), (10, 10, 2, True), (8, 2, 2, True), (8, 1, 5, False), (8, 1, 2, True)])
+def test_chunks_join_in_eager_calls_and_take_the_merge_launch_under_capture(heads, kv_heads, chunk_pages, joined):
+    """A captured call is the split and the merge launch, whatever the grid; an eager one of a small grid is one launch unless a block
+    would fold more than two heads. The same bits."""
+    from cuda.bindings import runtime as cudart
+
+    lens = [512, 500, 1]
+    case = helpers.attention_case(970 + heads + chunk_pages, heads, kv_heads, lens)
+    cache, q = load_cache(case, max(lens)), helpers.bits_bf16(case["q"]).cuda()
+    lens_t = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    out, captured = torch.zeros_like(q), torch.zeros_like(q)
+    states = torch.zeros(ncb.attention.workspace_bytes(3, heads, kv_heads, max(lens), chunk_pages), dtype=torch.uint8, device="cuda")
+    args = dict(max_kv_len=max(lens), chunk_pages=chunk_pages, workspace=states)
+    ncb.decode_attention(q, cache, lens_t, out=out, **args)
+    assert bool(states.any()) == (not joined)  # the states that a merge launch reads
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        ncb.decode_attention(q, cache, lens_t, out=captured, **args)
+    err, _, nodes = cudart.cudaGraphGetNodes(cudart.cudaGraph_t(graph.raw_cuda_graph()))
+    assert err == cudart.cudaError_t.cudaSuccess and nodes == 2
+    graph.replay()
+    assert torch.equal(out, captured) and bool(out.any()) and bool(states.any())
