@@ -55,14 +55,6 @@ def no_collection():
             gc.enable()
 
 
-def streamed(rows: int, N: int, K: int) -> bool:
-    """Whether stream_gemm has a pass of more than 64 rows rather than tile_gemm: deep and narrow products, whose tiles are few and each
-    as long as the whole depth, where stream_gemm splits the depth over clusters. us, tile_gemm -> stream_gemm: 100 rows, 1,280 wide,
-    K 3,072 15.6 -> 9.1, K 5,120 23.7 -> 10.9, 2,048 wide, K 5,120 24.2 -> 11.9; 200 rows, 1,280 wide 16.5 -> 11.2, 24.7 -> 13.0. Not K
-    1,280 (200 rows, 1,280 wide 8.9 -> 9.9; 3,840 wide 10.1 -> 12.1), nor, above 128 rows, 2,048 wide (24.9 -> 25.2)."""
-    return K >= 2048 and (rows <= 128 and N <= 4096 or rows <= 256 and N <= 1536)
-
-
 @dataclass
 class DecoderConfig:
     n_layers: int
@@ -548,7 +540,9 @@ class Decoder(StepDecoder):
         """epilogue(x . w^T) for a pass of any number of rows: x bf16 (rows, K), w bf16 (N, K); epilogue 0 store,
         2 relu^2, 3 fp32 output; resid (rows, N) bf16: resid += bf16(x . w^T) in place (epilogue 1), returned; out: a
         bf16 (rows, N) buffer to write into instead of a new tensor (the result is whatever is returned).
-        This package's tiled tcgen05 GEMM (csrc/tile_gemm.cu), or stream_gemm (streamed), when N is a multiple of 128 and K of 64; other shapes
+        This package's tiled tcgen05 GEMM (csrc/tile_gemm.cu) when N is a multiple of 128 and K of 64, whatever the number of rows: it adds
+        a row's k-blocks up in one order, so that a prompt's cache bytes do not depend on what shares its pass (stream_gemm, which
+        splits the depth, is faster for deep, narrow products of up to about 200 rows and adds in another order). Other shapes
         (toy models) go to torch's GEMM with the same epilogue applied afterwards."""
         rows, K, N = x.shape[0], x.shape[1], w.shape[0]
         if resid is not None:
@@ -557,11 +551,6 @@ class Decoder(StepDecoder):
         if self.use_tile_gemm and N % 128 == 0 and K % 64 == 0 and x.is_contiguous() and w.is_contiguous():
             y = resid if resid is not None else out if out is not None and epilogue != 3 else torch.empty(
                 (rows, N), dtype=torch.float32 if epilogue == 3 else torch.bfloat16, device=x.device)
-            if self.use_stream_gemm and streamed(rows, N, K):
-                check(cuda_library("stream_gemm").stream_gemm(pointer(x), pointer(w), None if resid is None else pointer(resid), pointer(y),
-                                                              rows, N, K, 0, epilogue, 0, None, 0, pointer(self.status), stream()),
-                      "stream_gemm")
-                return y
             check(cuda_library("tile_gemm").tile_gemm(pointer(x), pointer(w), None if resid is None else pointer(resid),
                                                       pointer(y), rows, N, K, epilogue, pointer(self.status), stream()),
                   "tile_gemm")

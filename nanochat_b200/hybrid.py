@@ -17,7 +17,7 @@ from dataclasses import dataclass
 import torch
 from torch import Tensor
 
-from .decoder import StepDecoder, streamed
+from .decoder import StepDecoder
 from .kv_cache import cache_pages
 from .mixers import MIXERS, RowPlan, Rows, pad_to, up
 from .native import MAX_STREAMS, GemmRs, check, cuda_library, pointer, stream
@@ -234,6 +234,15 @@ class HybridWeights:
                 state[p + "norm2"] = w(C, scale=0.1, base=around)
                 state.update({p + "mlp.gate": w(spec.ff, C), p + "mlp.up": w(spec.ff, C), p + "mlp.down": w(C, spec.ff)})
         return state
+
+
+def streamed(rows: int, N: int, K: int) -> bool:
+    """Whether stream_gemm has a pass of more than 64 rows rather than tile_gemm: deep and narrow products, whose tiles are few and each
+    as long as the whole depth, where stream_gemm splits the depth over clusters. us, tile_gemm -> stream_gemm: 100 rows, 1,280 wide,
+    K 3,072 15.6 -> 9.1, K 5,120 23.7 -> 10.9, 2,048 wide, K 5,120 24.2 -> 11.9; 200 rows, 1,280 wide 16.5 -> 11.2, 24.7 -> 13.0. Not K
+    1,280 (200 rows, 1,280 wide 8.9 -> 9.9; 3,840 wide 10.1 -> 12.1), nor, above 128 rows, 2,048 wide (24.9 -> 25.2). The two add a
+    row's products up in different orders, so a row's bits follow the number of rows in its pass."""
+    return K >= 2048 and (rows <= 128 and N <= 4096 or rows <= 256 and N <= 1536)
 
 
 class Stream:

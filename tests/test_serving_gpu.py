@@ -71,6 +71,21 @@ def test_long_prompts_among_short_ones_match_each_alone(kv_heads):
         assert int(got.status.item()) == 0 and all(torch.equal(g.pages, w.pages) for g, w in zip(got.caches, want.caches))
 
 
+def test_prompts_of_a_model_with_deep_products_keep_their_bits_in_any_pass():
+    """A down projection of depth 2,048: the same cache bytes whether a prompt has its pass to itself, shares one
+    with others or is cut over several."""
+    cfg = DecoderConfig(n_layers=3, hidden=512, n_heads=4, n_kv_heads=2, intermediate=2048, vocab=V, max_len=576)
+    w = DecoderWeights.random_init(cfg, seed=37, device="cuda", std=0.05)
+    prompts = [prompt(120 + i, n) for i, n in enumerate((61, 101, 201, 501, 3, 257))]
+    want = Decoder(cfg, w, len(prompts))
+    for b, p in enumerate(prompts):
+        want.prefill([p], [b])
+    for order, rows_per_pass in ((range(6), 4096), ([5, 3, 0, 4, 1, 2], 4096), (range(6), 200), (range(6), 70), ([3, 4, 2, 5, 1, 0], 330)):
+        got = Decoder(cfg, w, len(prompts))
+        got.prefill([prompts[b] for b in order], list(order), rows_per_pass=rows_per_pass)
+        assert int(got.status.item()) == 0 and all(torch.equal(g.pages, o.pages) for g, o in zip(got.caches, want.caches)), (list(order), rows_per_pass)
+
+
 def test_stopping_criteria_token_limits_and_masks():
     class Only:
         """Allows the tokens of a fixed set."""
