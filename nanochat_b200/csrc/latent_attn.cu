@@ -23,7 +23,6 @@
  */
 #include "attn_tiles.cuh"
 
-#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -497,25 +496,31 @@ template <typename T> __global__ void __launch_bounds__(THREADS) k_latent_out_an
     }
 }
 
-constexpr int OUT_THREADS = 256, OUT_ROWS = 4;
+constexpr int OUT_THREADS = 256;
 
-/* Grid (slices, heads, ceil(rows / 4)), cluster (slices, 1, 1): a block merges rank / slices latent columns of 4 rows,
+/* Threads of k_latent_out that share the states of one item (four latent columns of a row). */
+__host__ __device__ inline int out_shares(int rows, int items) {
+    const int fit = OUT_THREADS / items;
+    return rows > 8 || fit < 1 ? 1 : fit < 4 ? fit : 4;
+}
+
+/* Grid (slices, heads, ceil(rows / ROWS)), cluster (slices, 1, 1): a block merges rank / slices latent columns of ROWS rows (4 or 16),
  * multiplies them by its columns of W_uv (on their way to shared memory before the dependency wait) for all of the head's
- * values, and the cluster adds the partial products up. Bound by the chain of loads of the longest rows' states, so few rows share a
- * block and its weights (which come from L2) although the product's M is 16: 32 rows of 256 to 8,192 positions, longest first, 16
- * heads: 19.0 -> 13.5 us a launch (16 rows per block before). */
-__global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) {
+ * values, and the cluster adds the partial products up. A small grid is bound by the chain of loads of the longest rows' states, so
+ * that four rows share a block and its weights although the product's M is 16; a large one by the weights, which every block reads
+ * from L2 (latent_out has the line between them). */
+template <int ROWS> __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) {
     extern __shared__ __align__(128) uint8_t raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int slices = gridDim.x, rank_block = blockIdx.x, h = blockIdx.y, r0 = blockIdx.z * OUT_ROWS;
+    const int slices = gridDim.x, rank_block = blockIdx.x, h = blockIdx.y, r0 = blockIdx.z * ROWS;
     const int cols = a.rank / slices, c0 = rank_block * cols, xs = cols + 8, V = a.vdim;
-    const int items = OUT_ROWS * (cols / 4), shares = max(1, min(OUT_THREADS / items, 4)); /* threads that share an item's states */
-    float *w = reinterpret_cast<float *>(raw);                                          /* [4][max_chunks, a multiple of 4] */
-    float *sum = w + OUT_ROWS * ((a.max_chunks + 3) & ~3);                              /* [4][vdim + 4] partial products */
-    float4 *part = reinterpret_cast<float4 *>(sum + OUT_ROWS * (V + 4));                /* [shares - 1][items] */
-    bf16 *x = reinterpret_cast<bf16 *>(part + (shares - 1) * items);                    /* [4][cols + 8] merged latent */
-    bf16 *u = x + OUT_ROWS * xs;                                                        /* [vdim][cols + 8] */
-    __shared__ int n_chunks[OUT_ROWS];
+    const int items = ROWS * (cols / 4), shares = out_shares(ROWS, items);
+    float *w = reinterpret_cast<float *>(raw);                                          /* [ROWS][max_chunks, a multiple of 4] */
+    float *sum = w + ROWS * ((a.max_chunks + 3) & ~3);                                  /* [ROWS][vdim + 4] partial products */
+    float4 *part = reinterpret_cast<float4 *>(sum + ROWS * (V + 4));                    /* [shares - 1][items] */
+    bf16 *x = reinterpret_cast<bf16 *>(part + (shares - 1) * items);                    /* [ROWS][cols + 8] merged latent */
+    bf16 *u = x + ROWS * xs;                                                            /* [vdim][cols + 8] */
+    __shared__ int n_chunks[ROWS];
     {
         const int per = cols / 8;
         const bf16 *src = (const bf16 *)a.w_uv + (size_t)h * V * a.rank + c0;
@@ -524,33 +529,34 @@ __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) 
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int rows = (int)(a.rows - r0 < OUT_ROWS ? a.rows - r0 : OUT_ROWS);
+    const int rows = (int)(a.rows - r0 < ROWS ? a.rows - r0 : ROWS);
     const size_t state = (size_t)(a.rank + STATE_PAD);
     const int ws = (a.max_chunks + 3) & ~3;
-    if (warp < OUT_ROWS) { /* the factor of every chunk's state, a warp per row: 2^(m - M) / L with the sink in M and L */
-        const int r = warp;
+    constexpr int PER_ROW = ROWS > 8 ? OUT_THREADS / ROWS : 32;
+    if (tid < ROWS * PER_ROW) { /* the factor of every chunk's state, PER_ROW threads per row: 2^(m - M) / L with the sink in M and L */
+        const int r = tid / PER_ROW, j = tid % PER_ROW;
         int n = 0, slot;
         if (r < rows) n = cut_of(length_of(a, r0 + r, slot), a.chunk_tiles).n_chunks;
         const float *p = a.parts + ((size_t)(r0 + r) * a.heads + h) * a.max_chunks * state;
         const float sink = a.sink ? a.sink[h] * LOG2E : -INFINITY;
         float M = sink, L = 0.f;
-        for (int c = lane; c < n; c += 32) M = fmaxf(M, p[c * state]);
-        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        for (int c = lane; c < n; c += 32) {
+        for (int c = j; c < n; c += PER_ROW) M = fmaxf(M, p[c * state]);
+        for (int o = PER_ROW / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        for (int c = j; c < n; c += PER_ROW) {
             const float2 ml = *reinterpret_cast<const float2 *>(p + c * state);
             const float e = exp2f(ml.x - M);
             w[r * ws + c] = e;
             L = fmaf(e, ml.y, L);
         }
-        for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        for (int o = PER_ROW / 2; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
         if (a.sink) L += exp2f(sink - M);
         const float inv = n > 0 ? 1.f / L : 0.f;
-        for (int c = lane; c < n; c += 32) w[r * ws + c] *= inv;
-        if (lane == 0) n_chunks[r] = n;
+        for (int c = j; c < n; c += PER_ROW) w[r * ws + c] *= inv;
+        if (j == 0) n_chunks[r] = n;
     }
     __syncthreads();
     for (int at = tid; at < items * shares; at += OUT_THREADS) { /* (shares > 1: every thread has one item at most) */
-        const int i = at % items, share = at / items, r = i / (cols / 4), c4 = i % (cols / 4) * 4;
+        const int i = ROWS > 8 ? at : at % items, share = ROWS > 8 ? 0 : at / items, r = i / (cols / 4), c4 = i % (cols / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         const int n = n_chunks[r];
         const float *p = a.parts + ((size_t)(r0 + r) * a.heads + h) * a.max_chunks * state + STATE_PAD + c0 + c4;
@@ -580,17 +586,21 @@ __global__ void __launch_bounds__(OUT_THREADS) k_latent_out(const ncb_latent a) 
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int n0 = warp * 8; n0 < V; n0 += OUT_THREADS / 4) { /* 8 output values at a time; rows past the fourth are zeros */
+    for (int n0 = warp * 8; n0 < V; n0 += OUT_THREADS / 4) { /* 8 output values at a time; of 4 rows, those past the fourth are zeros */
         float acc[2][4] = {};
         const bf16 *wr = u + (n0 + g) * xs + 8 * t, *xl = x + g * xs + 8 * t;
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll 4
         for (int k = 0; k < cols; k += 32) {
-            const uint4 lo = g < OUT_ROWS ? *reinterpret_cast<const uint4 *>(xl + k) : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 lo = ROWS > 8 || g < ROWS ? *reinterpret_cast<const uint4 *>(xl + k) : zero;
+            const uint4 hi = ROWS > 8 ? *reinterpret_cast<const uint4 *>(xl + 8 * xs + k) : zero;
             const uint4 b = *reinterpret_cast<const uint4 *>(wr + k);
-            mma_bf16(acc[0], lo.x, 0u, lo.y, 0u, b.x, b.y);
-            mma_bf16(acc[1], lo.z, 0u, lo.w, 0u, b.z, b.w);
+            mma_bf16(acc[0], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+            mma_bf16(acc[1], lo.z, hi.z, lo.w, hi.w, b.z, b.w);
         }
-        if (g < OUT_ROWS) *reinterpret_cast<float2 *>(sum + g * (V + 4) + n0 + 2 * t) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+        float *s = sum + g * (V + 4) + n0 + 2 * t;
+        if (ROWS > 8 || g < ROWS) *reinterpret_cast<float2 *>(s) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+        if (ROWS > 8) *reinterpret_cast<float2 *>(s + 8 * (V + 4)) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
     }
     cg::cluster_group cluster = cg::this_cluster();
     if (slices > 1) cluster.sync();
@@ -881,6 +891,17 @@ int check(const ncb_latent &g) {
                ? NCB_ERR_ALIGN : NCB_OK;
 }
 
+int sm_count() {
+    int device = 0, count = 0;
+    return cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && count > 0 ? count : 148;
+}
+
+size_t out_smem(const ncb_latent &g, int rows, int cols) {
+    const int items = rows * (cols / 4);
+    return (size_t)rows * ((g.max_chunks + 3) / 4 * 4) * 4 + (size_t)rows * (g.vdim + 4) * 4 + (size_t)(out_shares(rows, items) - 1) * items * 16 +
+           (size_t)(rows + g.vdim) * (cols + 8) * 2;
+}
+
 template <int MK, int MN, int STAGES> int launch_split(const ncb_latent &g, cudaStream_t s) {
     CUtensorMap map;
     if (!tensor_map(g.cache, g.n_slots * g.capacity, g.rank + g.rot, TILE, &map)) return NCB_ERR_LAUNCH;
@@ -942,11 +963,17 @@ int latent_out(const ncb_latent *g, int f32, void *stream) {
     if (!f32) {
         int slices = 4;
         while (slices > 1 && g->rank % (slices * 32)) slices /= 2;
-        const int cols = g->rank / slices, items = OUT_ROWS * (cols / 4), shares = std::max(1, std::min(OUT_THREADS / items, 4));
-        const size_t smem = (size_t)OUT_ROWS * ((g->max_chunks + 3) / 4 * 4) * 4 + (size_t)OUT_ROWS * (g->vdim + 4) * 4 + (size_t)(shares - 1) * items * 16 +
-                            (size_t)(OUT_ROWS + g->vdim) * (cols + 8) * 2;
-        if (smem <= 200 * 1024)
-            return launch(k_latent_out, dim3(slices, g->heads, (unsigned)((g->rows + OUT_ROWS - 1) / OUT_ROWS)), smem, OUT_THREADS, slices, s, *g);
+        /* Four rows to a block while the GPU holds all blocks at once (about four to an SM, in clusters of four), else sixteen, whose
+         * blocks read W_uv four times less often. us a layer, sixteen -> four, 10 heads: 32 rows at 500 positions (320 blocks of four)
+         * 34.8 -> 29.2, 52 rows (520) at 64 26.6 -> 26.1, at 500 38.4 -> 33.8; 56 rows (560) 27.1 -> 31.2, 38.9 -> 39.4; 16 heads: 32 rows
+         * (512) 27.6 -> 26.1, 36.9 -> 31.2; 36 (576) 27.7 -> 31.2, 37.4 -> 37.9; 96 34.3 -> 45.6, 47.1 -> 57.9. */
+        const bool few = 2 * (long long)slices * g->heads * ((g->rows + 3) / 4) <= 7 * sm_count();
+        for (int rows : {few ? 4 : 16, 4}) { /* (four also where sixteen rows' factors do not fit) */
+            const size_t smem = out_smem(*g, rows, g->rank / slices);
+            if (smem > 200 * 1024) continue;
+            const dim3 grid(slices, g->heads, (unsigned)((g->rows + rows - 1) / rows));
+            return rows == 4 ? launch(k_latent_out<4>, grid, smem, OUT_THREADS, slices, s, *g) : launch(k_latent_out<16>, grid, smem, OUT_THREADS, slices, s, *g);
+        }
     }
     const size_t smem = ((size_t)g->max_chunks + g->rank) * sizeof(float);
     if (smem > 200 * 1024) return NCB_ERR_UNSUPPORTED;

@@ -112,6 +112,16 @@ def test_latent_attention_alone(dtype, sizes, mode):
     close(got, want, dtype)
 
 
+@pytest.mark.parametrize("sizes, pieces", [("rank 512", [32, 33, 17]), ("two head tiles", [112, 116, 5])])
+def test_latent_rows_in_blocks_of_four_and_sixteen(sizes, pieces):
+    """latent_out on both sides of the line between four and sixteen rows to a block (148 SMs: 518 blocks), with rows left over."""
+    entry = LATENT_SIZES[sizes]
+    state = cases.random_state(cases.config([entry], width=64), 7)
+    h = torch.randn(sum(pieces), 64, generator=torch.Generator().manual_seed(9)).to(BF16)
+    want = oracle.latent_attention(h.double(), oracle.part(state, "l0.mix."), entry["mixer"], 1e-5)
+    close(run_mixer(LatentAttention, entry, state, h, BF16, pieces, mode="absorbed"), want, BF16)
+
+
 @DTYPES
 @pytest.mark.parametrize("mode", ["absorbed", "expanded", "decoded"])
 def test_a_key_that_stands_out_is_found_wherever_it_lies(dtype, mode):
