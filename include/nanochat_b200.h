@@ -569,7 +569,7 @@ typedef struct {
 } ncb_gqa;
 int gqa_rows(const ncb_gqa *args, int f32, void *stream);
 int gqa_split_fused(int dim, int vdim);
-int gqa_split_blocks(int heads, int kv_heads, int dim, int vdim); /* blocks of gqa_split per SM that a choice of chunk_tiles may count on */
+int gqa_split_blocks(int heads, int kv_heads, int dim, int vdim); /* blocks per SM of gqa_split_fused sizes in bf16: what a choice of chunk_tiles may count on */
 int gqa_split(const ncb_gqa *args, int f32, void *stream);
 int gqa_merge(const ncb_gqa *args, int f32, void *stream);
 int gqa_prefill_supported(int dim, int vdim);

@@ -949,8 +949,12 @@ int gqa_rows(const ncb_gqa *g, int f32, void *stream) {
 /* 1 if gqa_split in bf16 takes these (padded) sizes with q NULL. */
 int gqa_split_fused(int dim, int vdim) { return dim > 0 && vdim > 0 && dim <= 256 && vdim <= 256; }
 
-/* Blocks of the fused form per SM, as far as registers go (see k_gqa_split): what a plan of chunks may count on. */
-int gqa_split_blocks(int heads, int kv_heads, int dim, int vdim) { return heads / kv_heads <= 8 && dim <= 128 && vdim <= 128 ? 3 : 2; }
+/* Blocks of the fused form per SM, as far as registers and two stages of shared memory go (see k_gqa_split): what a plan of chunks may
+ * count on. */
+int gqa_split_blocks(int heads, int kv_heads, int dim, int vdim) {
+    if (dim > 128 || vdim > 128) return split_smem(dim, vdim, 2).total <= 112 * 1024 ? 2 : 1;
+    return heads / kv_heads <= 8 ? 3 : 2;
+}
 
 int gqa_split(const ncb_gqa *g, int f32, void *stream) {
     if (!g) return NCB_ERR_ARG;

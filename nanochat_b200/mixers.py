@@ -265,6 +265,12 @@ class GroupedAttention:
         self.tiled = bf and bool(lib.gqa_prefill_supported(self.dim, self.vdim))
         self.wide = self.tiled and self.scale > 0.0 and bool(lib.gqa_prefill_tiles_supported(self.dim, self.vdim))
         self.tiled_f32 = not bf and bool(lib.gqa_prefill_f32_supported(self.dim, self.vdim))
+        # the split kernel's blocks per chunk of a row, and how many of them an SM holds: a block of the form for 32 bits and any sizes has
+        # one head. That form planned as the other (two or three blocks per SM, their heads together) was 9 or 6 % off its best chunk size
+        # (6 heads: 32 rows at 1,024 positions 166 or 197 us a layer, now 155; 8 at 4,096 207 or 164, now 133), planned like this 0.5 %
+        # (205 batches of 1 to 32 rows).
+        self.blocks_per_chunk = G * ((H // G + 15) // 16) if self.fused else H
+        self.split_blocks = lib.gqa_split_blocks(self.heads, self.kv_heads, self.dim, self.vdim) if self.fused else 8
 
     ROW_TILE = 64     # rows per tile of gqa_prefill
     WIDE_TILE = 128   # rows per tile of gqa_prefill_tiles
@@ -293,17 +299,28 @@ class GroupedAttention:
         return (ring + (up(max_len, 64) * G * (dim + vdim) if own else 0)) * itemsize
 
     def chunk_for(self, lens: "list[int]", most: int) -> int:
-        """Tiles per chunk of the split kernel for rows of these lengths, at most 128 chunks for `most` positions: enough blocks
-        to fill the GPU (gqa_split_blocks per SM), chunks long enough to be worth a state."""
+        """Tiles per chunk of the split kernel for rows of these lengths, at most 128 chunks for `most` positions: the size with the
+        least modelled time, rounds of the blocks that fit the GPU (split_blocks per SM) times a block's tiles plus a fixed cost.
+        With three blocks to an SM a round that fills them is 1.25 times as long, and what many chunks cost elsewhere counts: the longest
+        row's states in the merge, the places of blocks past the end of shorter rows (in tiles; fitted to 265 batches of 1 to 64 equal and
+        ragged rows of 32 to 8,192 positions at 1 to 12 key/value heads and all chunk sizes, on average 2 % off the best size). Two
+        blocks' places for all of them left 3 % (16 heads over 4: 32 x 4,096 69 us a layer, now 61), three without these terms lost
+        as much again (64 x 512 33 -> 43, now 33; 8 heads of 64, 2 rows of 8,192 and 256 22 -> 29, now 22)."""
         tiles = np.maximum((np.asarray(lens, dtype=np.int64) + GQA_TILE - 1) // GQA_TILE, 1)
-        top, least = int(tiles.max()), max(8, ((most + GQA_TILE - 1) // GQA_TILE + 127) // 128)
-        per_chunk = self.kv_heads * ((self.heads // self.kv_heads + 15) // 16)
-        places = SM_COUNT * cuda_library("gqa_attn").gqa_split_blocks(self.heads, self.kv_heads, self.dim, self.vdim)
+        all_tiles, top = (most + GQA_TILE - 1) // GQA_TILE, int(tiles.max())
+        least = max(8, (all_tiles + 127) // 128)
+        places = SM_COUNT * self.split_blocks
         best, cost = least, float("inf")
         c = least
         while c < 2 * max(top, least):
-            blocks = int(((tiles + c - 1) // c).sum()) * per_chunk
-            now = -(-blocks // places) * (min(c, top) + 8.0)
+            blocks = int(((tiles + c - 1) // c).sum()) * self.blocks_per_chunk
+            if self.split_blocks == 3:
+                full, rest = divmod(blocks, places)
+                rounds = 1.25 * (full + (rest > 2 * SM_COUNT)) + (0 < rest <= 2 * SM_COUNT)
+                idle = -(-all_tiles // c) * len(tiles) * self.blocks_per_chunk - blocks
+                now = rounds * (min(c, top) + 16.0) + 0.4 * -(-top // c) + idle / SM_COUNT
+            else:
+                now = -(-blocks // places) * (min(c, top) + 8.0)
             if now < cost:
                 best, cost = c, now
             c += max(1, c // 8)

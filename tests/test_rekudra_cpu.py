@@ -313,3 +313,22 @@ def test_sizes_of_the_chunked_delta_rule():
     lib = native.cuda_library("delta_rule")
     assert lib.delta_chunk_tokens(128, 128, 4, 128, 128) == 64 and lib.delta_chunk_tokens(256, 256, 4, 128, 128) == 32
     assert lib.delta_chunk_tokens(272, 64, 4, 16, 16) == 0 and lib.delta_chunk_tokens(128, 128, 4, 4096, 16) == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,dtype,blocks,per_sm", [
+    (16, 4, 128, torch.bfloat16, 4, 3), (36, 2, 128, torch.bfloat16, 4, 2), (8, 2, 192, torch.bfloat16, 2, 2), (8, 2, 256, torch.bfloat16, 2, 1),
+    (6, 6, 128, torch.float32, 6, 8), (12, 2, 128, torch.float32, 12, 8), (4, 2, 272, torch.bfloat16, 4, 8)])
+def test_chunk_plans_count_the_blocks_of_the_kernel_that_runs(heads, kv_heads, dim, dtype, blocks, per_sm):
+    """Blocks of a chunk and blocks per SM: of the form that keeps a key/value head's query heads together by registers and shared memory,
+    of the form for 32 bits and any sizes (a block has one head) otherwise. Plans cover every length in at most 128 chunks."""
+    layer = cases.attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, rot_dims=16)
+    state = cases.random_state(cases.config([layer], width=64), 3)
+    mixer = GroupedAttention(layer["mixer"], {k[len("l0.mix."):]: v for k, v in state.items() if k.startswith("l0.mix.")}, 1e-5, 128, dtype, "cpu")
+    assert (mixer.blocks_per_chunk, mixer.split_blocks) == (blocks, per_sm)
+    for lens, most in (([1], 64), ([8192], 8192), ([512] * 64, 512), ([8192, 256], 8192), ([1024, 181, 32], 8192), ([20000, 5], 32768)):
+        chunk = mixer.chunk_for(lens, most)
+        assert chunk >= 8 and -(-(-(-most // 16)) // chunk) <= 128
+    if per_sm == 3:  # short rows in one piece each, one long row not in more pieces than its merge is worth
+        assert mixer.chunk_for([512] * 64, 512) >= 32 and -(-512 // mixer.chunk_for([8192, 256], 8192)) <= 70
+    if dtype == torch.float32:  # one round of the blocks that fit, where two rounds of larger ones were planned
+        assert -(-64 // mixer.chunk_for([1024] * 32, 1024)) * 32 * heads <= 8 * 148 and mixer.chunk_for([4096] * 8, 4096) < 256 / 4
