@@ -331,6 +331,17 @@ class GroupedAttention:
             self._chunks[rows, max_len] = self.chunk_for([max_len] * rows, max_len)
         return self._chunks[rows, max_len]
 
+    def shares_keys(self, plan: RowPlan) -> bool:
+        """Whether gqa_prefill_f32 has a 32-bit pass. A tile walks through all its keys in one block, which the split kernel cuts up: it
+        takes 32 tiles' worth of the longest walk (256 pairs of a row and a position per position) to pay for that. us a layer, split and
+        merge -> tiles, 6 heads: 8 rows at the start 24 -> 25, behind 1,000 positions 53 -> 129, behind 4,000 98 -> 434; 32 rows behind 1,000
+        97 -> 137; 64 behind 200 63 -> 59, behind 4,000 489 -> 444; 300 at the start 126 -> 63; 12 heads: 16 behind 1,000 96 -> 134; 32
+        150 -> 137; one of 100 beside 15 rows behind 2,000 246 -> 283."""
+        def pays():
+            _, longest, pairs = plan.extent()
+            return plan.longest >= self.TILED_FROM and pairs * self.heads >= 32 * self.F32_TILE * longest and plan.row_tiles(self.F32_TILE)[1] <= 65535
+        return self.tiled_f32 and plan.once(("shares_keys", self.heads), pays)
+
     def run(self, proj: Tensor, cache: AttentionCache, rows: Rows, out: "Tensor | None") -> None:
         n, f32, lib, kv = rows.n, int(self.dtype == torch.float32), cuda_library("gqa_attn"), cache.kv
         a = Gqa(conv=self.conv.args(proj, cache.ring, rows), kv=kv.rows.data_ptr(), off_q=self.off_q, off_k=self.off_k, off_v=self.off_v,
@@ -351,8 +362,7 @@ class GroupedAttention:
                 a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
                 entry = "gqa_prefill_tiles" if wide else "gqa_prefill"
                 check(getattr(lib, entry)(pointer_to(a), stream()), entry)
-        elif (out is not None and self.tiled_f32 and rows.plan is not None and rows.plan.longest >= self.TILED_FROM
-              and rows.plan.row_tiles(self.F32_TILE)[1] <= 65535):
+        elif out is not None and rows.plan is not None and self.shares_keys(rows.plan):
             tiles, a.n_tiles = rows.plan.row_tiles(self.F32_TILE)
             a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
             check(lib.gqa_prefill_f32(pointer_to(a), stream()), "gqa_prefill_f32")

@@ -332,3 +332,16 @@ def test_chunk_plans_count_the_blocks_of_the_kernel_that_runs(heads, kv_heads, d
         assert mixer.chunk_for([512] * 64, 512) >= 32 and -(-512 // mixer.chunk_for([8192, 256], 8192)) <= 70
     if dtype == torch.float32:  # one round of the blocks that fit, where two rounds of larger ones were planned
         assert -(-64 // mixer.chunk_for([1024] * 32, 1024)) * 32 * heads <= 8 * 148 and mixer.chunk_for([4096] * 8, 4096) < 256 / 4
+
+
+@pytest.mark.parametrize("heads,kv_heads,runs,shared", [
+    (6, 6, [(0, 300)], True), (6, 6, [(0, 8)], False), (6, 6, [(1000, 8)], False), (6, 6, [(4000, 32)], False), (6, 6, [(200, 64)], True),
+    (6, 6, [(4000, 64)], True), (12, 2, [(1000, 16)], False), (12, 2, [(1000, 32)], True), (6, 6, [(1000, 16)] * 8, True),
+    (6, 6, [(0, 100)] + [(2000, 1)] * 15, False), (12, 2, [(0, 7)] * 90, False)])
+def test_short_32_bit_portions_behind_long_contexts_are_split(heads, kv_heads, runs, shared):
+    """Where eight rows of a 32-bit pass share their keys: by how much work there is for each step of the longest walk, as measured."""
+    layer = cases.attention(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, rot_dims=16)
+    state = cases.random_state(cases.config([layer], width=64), 3)
+    mixer = GroupedAttention(layer["mixer"], {k[len("l0.mix."):]: v for k, v in state.items() if k.startswith("l0.mix.")}, 1e-5, 128, torch.float32, "cpu")
+    slots, positions = [s for s, (_, n) in enumerate(runs) for _ in range(n)], [p for at, n in runs for p in range(at, at + n)]
+    assert mixer.shares_keys(RowPlan(slots, positions, "cpu")) == shared
