@@ -770,14 +770,14 @@ template <int NV> __global__ void __launch_bounds__(THREADS) k_gqa_prefill_f32(c
     float *q = shared, *k = q + F32_ROWS * a.dim, *v = k + 2 * F32_KEYS * ks, *p = v + 2 * F32_KEYS * a.vdim;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int row0 = a.tile_row[tile], rows = min(a.tile_rows[tile], F32_ROWS), pos0 = a.tile_pos[tile];
-    int slot = 0, end;
-    const bool ok = rows > 0 && length_of(a, row0, slot) > 0 && length_of(a, row0 + rows - 1, end) == pos0 + rows; /* flagged by gqa_rows too */
+    const int row0 = a.tile_row[tile], listed = min(a.tile_rows[tile], F32_ROWS), pos0 = a.tile_pos[tile];
+    int slot = 0;
+    const bool ok = lane < listed && length_of(a, row0 + lane, slot) == pos0 + lane + 1 && pos0 >= 0; /* a row outside the cache is flagged */
+    const int rows = __ffs(~__ballot_sync(0xffffffffu, ok)) - 1; /* rows from there on get zeros, those before it are whole */
+    slot = __shfl_sync(0xffffffffu, slot, 0);
     float *out = (float *)a.out + (size_t)row0 * a.ldo + h * a.vdim;
-    if (!ok) {
-        for (int i = tid; i < rows * a.vdim; i += THREADS) out[(size_t)(i / a.vdim) * a.ldo + i % a.vdim] = 0.f;
-        return;
-    }
+    for (int i = rows * a.vdim + tid; i < listed * a.vdim; i += THREADS) out[(size_t)(i / a.vdim) * a.ldo + i % a.vdim] = 0.f;
+    if (rows == 0) return;
     const float *cache = cache_row<float>(a, slot, h / (a.heads / a.kv_heads), 0);
     const int keys = pos0 + rows, n = (keys + F32_KEYS - 1) / F32_KEYS;
     auto fetch = [&](int i) { /* positions past the tile's last row are zeros */

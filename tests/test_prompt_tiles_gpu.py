@@ -387,3 +387,33 @@ def test_grouped_in_32_bits(heads, kv_heads, dim, vdim, runs):
         if seen < count:
             assert not torch.isfinite(got[row + count - 1]).any()
         row += count
+
+
+def test_grouped_in_32_bits_answers_the_rows_before_a_refused_one():
+    """A portion that runs over the end of the rotary table: rows up to it are what they are without the others, the rest are zeros and flagged."""
+    gen = torch.Generator(device="cuda").manual_seed(76)
+    heads, kv_heads, dim, vdim, capacity, table = 4, 2, 32, 48, 192, 133
+    ldp, pos = heads * dim, list(range(120, 141))
+    n, good = len(pos), table - 120
+    q, proj = torch.randn(n, heads, dim, generator=gen, device="cuda"), torch.randn(n, ldp, generator=gen, device="cuda")
+    kv = torch.randn(2, kv_heads, capacity, dim + vdim, generator=gen, device="cuda")
+    ring, taps, lib = torch.zeros(2, 1, ldp, device="cuda"), torch.ones(1, ldp, device="cuda"), cuda_library("gqa_attn")
+
+    def attend(count, slot):
+        dev = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos[:count], [slot] * count)]
+        status, out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((count, heads * vdim), 7.0, device="cuda")
+        a = Gqa(conv=Conv(proj=proj.data_ptr(), ring=ring.data_ptr(), w=taps.data_ptr(), rows=count, ldp=ldp, taps=1, width=ldp, n_slots=2,
+                          pos=dev[0].data_ptr(), slot_map=dev[1].data_ptr()), q=q.data_ptr(), kv=kv.data_ptr(), out=out.data_ptr(), ldo=out.stride(0),
+                heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, norm_count=dim, capacity=capacity, table_len=table, scale=dim ** -0.5, eps=1e-6,
+                status=status.data_ptr())
+        tiles, a.n_tiles = RowPlan([slot] * count, pos[:count], "cuda").row_tiles(8)
+        a.tile_row, a.tile_rows, a.tile_pos = (tiles[i].data_ptr() for i in (0, 1, 3))
+        check(lib.gqa_prefill_f32(ctypes.byref(a), stream()), "gqa_prefill_f32")
+        return out, int(status.item())
+
+    want, flags = attend(good, 1)
+    assert flags == 0 and bool(want.any())
+    got, flags = attend(n, 1)
+    assert flags != 0 and torch.equal(got[:good], want) and not got[good:].any()
+    got, flags = attend(n, 2)  # a slot that is not there
+    assert flags != 0 and not got.any()
