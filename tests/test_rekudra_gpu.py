@@ -115,6 +115,20 @@ def test_attention_alone(dtype, sizes, mode):
     close(run_mixer(mixer, fresh_cache(mixer, n), h, dtype, pieces), want, dtype)
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(9, 1, 128, 112), (20, 1, 80, 128), (8, 1, 128, 128), (16, 1, 64, 64), (12, 1, 160, 256), (18, 2, 256, 144), (7, 1, 256, 32)])
+@pytest.mark.parametrize("mode", ["rows", "decoded"])
+def test_more_and_fewer_than_eight_heads_of_a_key(heads, kv_heads, dim, vdim, mode):
+    """k_gqa_split with and without the upper half of its MMAs' rows, at every width it is instantiated for."""
+    entry, n, C = cases.attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, rot_dims=32, scale=0.2), 90, 64
+    state = cases.random_state(cases.config([entry], width=C), 27)
+    h = torch.randn(n, C, generator=torch.Generator().manual_seed(28)).to(BF16)
+    w = oracle.part(state, "l0.mix.")
+    want = oracle.attention(h.double(), w, entry["mixer"], 1e-5, oracle.keys_and_values(h.double(), w, entry["mixer"], 1e-5))
+    mixer = new_mixer(GroupedAttention, entry, state, BF16, 128)
+    mixer.tiled = False
+    close(run_mixer(mixer, fresh_cache(mixer, n), h, BF16, [33, 2, n - 35] if mode == "rows" else [1] * n), want, BF16)
+
+
 @DTYPES
 @pytest.mark.parametrize("mode", ["tiled", "rows", "decoded"])
 def test_a_key_that_stands_out_is_found_wherever_it_lies(dtype, mode):
