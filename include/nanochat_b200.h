@@ -412,15 +412,15 @@ int stream_gemm_mix(const void *x, const void *w, const void *resid, const void 
                     void *stream);
 
 /* ---- library tile_gemm --------------------------------------------------------------------------------------
- * The same GEMM for any number of rows as a tiled tcgen05 kernel (128 rows x 256 features per tile, TMA-staged operands,
- * two accumulators in tensor memory so that the epilogue of one tile overlaps the MMAs of the next, one persistent
- * block per SM): the GEMMs of prefill passes and of decode steps above 64 sequences, where the reference runs k_wgmma
+ * The same GEMM for any number of rows as a tiled tcgen05 kernel (tiles of 128 x 128, 128 x 256, or 256 x 256 and 256 x 320 for
+ * a pair of blocks; TMA-staged operands, accumulators in tensor memory, two where they fit so that the epilogue of one tile
+ * overlaps the MMAs of the next, one persistent block per SM): the GEMMs of prefill passes and of decode steps above 64 sequences, where the reference runs k_wgmma
  * over prompt rows (model/kernels/decode.cu:232-359,1041-1051). */
 
 /*
  * y = epilogue(x . W^T). x bf16 [rows][K]; w bf16 [N][K]; y bf16 [rows][N] (fp32 for epilogue 3); resid bf16 [rows][N]
  * for epilogue 1 (may be y itself). epilogue: 0 store, 1 residual add (in bf16, after rounding the product), 2 relu^2,
- * 3 fp32 store. Any rows >= 0; N a multiple of 128 (tiles are 256 wide when N is a multiple of 256); K a multiple of
+ * 3 fp32 store. Any rows >= 0; N a multiple of 128 (see tile_gemm_form for the tiles it gets); K a multiple of
  * 64; all pointers 16-byte aligned. No fused input norm: passes of this size keep the normed rows in memory
  * (add_rms_norm). status: optional device word for NCB_DEV_WAIT_TIMEOUT. Launched with programmatic stream
  * serialisation.
@@ -433,7 +433,8 @@ int tile_gemm(const void *x, const void *w, const void *resid, void *y, long lon
  * pair of blocks on neighbouring SMs per 256 x 256 or 256 x 320 tile (tcgen05 cta_group::2: each block stages its own
  * 128 rows of x and half of the W tile, so a block loads a third less per product; the 320-wide tile is taken where it
  * makes fewer, fuller rounds, e.g. N = 1280); N must be a multiple of 256 or 640, else NCB_ERR_UNSUPPORTED. form 0:
- * tile_gemm's own choice (pairs where they apply and rows > 128). All forms give the same bits. No counterpart in the
+ * tile_gemm's own choice: 128 x 128 tiles of form 1 where one round of the SMs takes all of them, else form 2 where it applies and
+ * rows > 128, else form 1. All forms give the same bits. No counterpart in the
  * reference (its GEMM is one kernel form).
  */
 int tile_gemm_form(const void *x, const void *w, const void *resid, void *y, long long rows, int N, int K, int epilogue,

@@ -224,7 +224,7 @@ class PrefillPlan:
     #   32 / 8    1 x 256  23.2 -> 17.3   8 x 256 52.4 -> 51.0   8 x 512 137 -> 100     16 x 100 36.6 -> 42.5    1 x 4096 621 -> 230
     #   16 / 2    1 x 256  21.8 -> 16.4   8 x 256 29.6 -> 27.5   8 x 512 69.2 -> 48.9   16 x 100 19.9 -> 24.7    1 x 4096 317 -> 116
     # (A single prompt of 256 to 383 rows with equal heads would gain, eight of them would lose, and a row's kernel must not depend on
-    # the others.)
+    # the others. At 512 rows eight prompts of 10 heads are level: 53.4 and 54.2 above, 54.8 and 53.8 with L2 flushed; one is 38.9 -> 27.1.)
     WIDE_ROWS = 64                # rows of a portion
     WIDE_PAIRS = 6 * 1024         # per page and query head: about 96 positions a row
     WIDE_GROUP_PAIRS = 12 * 1024  # per page and key/value head

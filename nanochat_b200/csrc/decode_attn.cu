@@ -53,7 +53,7 @@ constexpr float P_SCALE = 256.f;          /* folded probabilities in (0, 1] -> e
 constexpr float LO_SCALE = 16.f;          /* second term's gain: the first term's rounding error is <= 2^-4 ulp-wise */
 constexpr float MIN_LOG2_VSCALE = -64.f;
 constexpr size_t ATTN_SMEM = (size_t)WARPS * PAGE_BYTES;
-static_assert(WARPS * 4 * 2 * PART * sizeof(float) <= ATTN_SMEM, "the merge area reuses the ring");
+static_assert((WARPS + 1) * 4 * 2 * PART * sizeof(float) <= ATTN_SMEM, "the merge area, and a joined block's states behind it, reuse the ring");
 static_assert(THREADS >= HEAD_DIM && 12 % WARPS == 0, "the final merge maps one thread to one output dim");
 
 struct AttnArgs {
@@ -72,8 +72,8 @@ struct AttnArgs {
     long long qkv_row_stride;
     int table_len;
     ValueEmbed ve; /* APPEND only; table == NULL: the layer has no value embedding */
-    bf16 *direct;  /* one chunk per sequence (max_chunks == 1): the block normalises and writes out[B][Hq][128] itself */
-    int joined;            /* a sequence's chunks are one cluster, which merges their states itself; `direct` is set */
+    bf16 *direct;  /* one chunk per sequence (max_chunks == 1), or joined: the blocks normalise and write out[B][Hq][128] themselves */
+    int joined;    /* a sequence's chunks are one cluster, which merges their states; `direct` is set */
 };
 
 /* ---- PTX wrappers ------------------------------------------------------------------------------------------- */

@@ -14,6 +14,8 @@
  * K 1920 93 -> 35, N 768 K 768 39 -> 17; one row, N 768 K 1920 84 -> 6.3, N 65536 K 768 188 -> 52 (3.9 TB/s); 1024 rows, N 4096 K 1024
  * 254 -> 213 (40 TFLOP/s: a thread's 16 loads of 16 bytes per 128 paired multiply-adds keep shared memory as busy as the FMA pipe).
  * One block of 256 threads per SM: 76, 33, 16, 6.7, 72, 223.
+ * The tile's height and the split follow the number of rows, and with them the order in which a row's products are added up: a row's last
+ * bits follow its pass.
  */
 #include "gemm_rs.cuh"
 

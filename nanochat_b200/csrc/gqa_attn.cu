@@ -368,7 +368,7 @@ __host__ __device__ inline SplitSmem split_smem(int dim, int vdim, int stages) {
 /* Grid (max chunks, kv_heads x tiles of 16 query heads, rows). DK, VN: upper bounds of dim / 16 and vdim / 16. UPPER: a block has more than
  * eight heads; else the upper half of the MMAs' rows is zero and nothing is computed for it, which leaves registers for three blocks per
  * SM: every warp waits on its own chain of products and exponentials, so more warps are what helps. 16 heads over 4, batch 32 of 256 to
- * 8,192 positions, 16 layers: a step 2,948 -> 2,742 us (without the upper half alone 2,948). */
+ * 8,192 positions, 16 layers: a step 2,967 -> 2,712 us (leaving the upper half out with two blocks per SM gained nothing). */
 template <int DK, int VN, bool UPPER> __global__ void __launch_bounds__(THREADS, DK + VN > 16 ? 1 : UPPER ? 2 : 3) k_gqa_split(const ncb_gqa a, int stages) {
     extern __shared__ __align__(128) uint8_t raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, row = blockIdx.z;
@@ -761,8 +761,8 @@ __host__ __device__ inline int f32_smem(int dim, int vdim) { return F32_ROWS * d
 
 /* Grid (heads, row tiles): at most 8 consecutive rows of a sequence against its keys, 32 at a time, everything in fp32. k_gqa_split_any
  * reads all keys and values from L2 for every row (bound by that: 2.8 TB/s); here eight rows share them. Scores: a lane has a key, a
- * warp two rows. Values: a thread has NV columns of all rows. One sequence of 300 rows, 6 heads of 128, split and merge -> this:
- * 108 -> 45 us a layer. */
+ * warp two rows. Values: a thread has NV columns of all rows. One sequence of 300 rows, 6 heads of 128, split and merge -> this, with
+ * the rows' preparation: 126 -> 58 us a layer. */
 template <int NV> __global__ void __launch_bounds__(THREADS) k_gqa_prefill_f32(const ncb_gqa a) {
     extern __shared__ __align__(16) float shared[];
     __shared__ float shrink[F32_ROWS], sums[F32_ROWS];

@@ -639,7 +639,8 @@ class Decoder(StepDecoder):
                    choose: bool = True, slots: "list[int] | None" = None) -> Tensor:
         """One step on this package's kernels (GEMMs: see gemm_kernel): fp32 logits in buf["logits"]; with `choose`, tokens
         become the greedy choices and pos advances by one. 6 launches per layer: qkv GEMM (norm fused), split
-        attention (append fused), merge, o GEMM + residual, up GEMM (norm fused) + relu^2, down GEMM + residual."""
+        attention (append fused), merge, o GEMM + residual, up GEMM (norm fused) + relu^2, down GEMM + residual; no merge where a
+        sequence is one chunk, or a few that join (eager calls of small batches)."""
         cfg, lib, s = self.cfg, cuda_library("decode_step"), stream()
         rows, C, Fd, A = tokens.shape[0], cfg.hidden, cfg.intermediate, cfg.n_heads * HEAD_DIM
         workspace = self._workspace(rows, max_kv_len)

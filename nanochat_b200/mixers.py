@@ -334,9 +334,9 @@ class GroupedAttention:
     def shares_keys(self, plan: RowPlan) -> bool:
         """Whether gqa_prefill_f32 has a 32-bit pass. A tile walks through all its keys in one block, which the split kernel cuts up: it
         takes 32 tiles' worth of the longest walk (256 pairs of a row and a position per position) to pay for that. us a layer, split and
-        merge -> tiles, 6 heads: 8 rows at the start 24 -> 25, behind 1,000 positions 53 -> 129, behind 4,000 98 -> 434; 32 rows behind 1,000
-        97 -> 137; 64 behind 200 63 -> 59, behind 4,000 489 -> 444; 300 at the start 126 -> 63; 12 heads: 16 behind 1,000 96 -> 134; 32
-        150 -> 137; one of 100 beside 15 rows behind 2,000 246 -> 283."""
+        merge -> tiles, 6 heads: 8 rows at the start 24 -> 25, behind 1,000 positions 53 -> 113, behind 4,000 98 -> 377; 32 rows behind 1,000
+        97 -> 121; 64 behind 200 63 -> 54, behind 4,000 489 -> 386; 300 at the start 126 -> 58; 12 heads: 16 behind 1,000 96 -> 118; 32
+        150 -> 121; one of 100 beside 15 rows behind 2,000 246 -> 256."""
         def pays():
             _, longest, pairs = plan.extent()
             return plan.longest >= self.TILED_FROM and pairs * self.heads >= 32 * self.F32_TILE * longest and plan.row_tiles(self.F32_TILE)[1] <= 65535
